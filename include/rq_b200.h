@@ -51,7 +51,7 @@ typedef enum rq_status {
 #define RQ_MAX_RANKS 8   /* ranks of one node whose output buffers a push call can address */
 
 /* which kernel-side layouts rq_w4a4_prepare builds */
-#define RQ_PREPACK_DECODE  1   /* int4 stream for the M <= 16 GEMV            (K*N/2 bytes) */
+#define RQ_PREPACK_DECODE  1   /* int4 stream, up to 64 tokens at a time       (K*N/2 bytes) */
 #define RQ_PREPACK_PREFILL 2   /* int8 operand for the tcgen05 GEMM           (K*N bytes)   */
 #define RQ_PREPACK_ALL     3
 
@@ -61,7 +61,7 @@ typedef enum rq_status {
 #define RQ_FMT_E4M3 1
 
 /* kernel selection of rq_w4a4_mul_mat */
-#define RQ_PATH_AUTO  0        /* M <= 64: GEMV in passes of 16 tokens; else tcgen05 GEMM if prepacked for it */
+#define RQ_PATH_AUTO  0        /* M <= 64: from the int4 stream; else tcgen05 GEMM if prepacked for it */
 #define RQ_PATH_GEMV  1
 #define RQ_PATH_TC    2
 

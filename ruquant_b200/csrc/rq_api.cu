@@ -127,6 +127,7 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_prepare(const void
     // rq_info, patch:2027-2043): sum -> weight-group mode, pad[0] -> Hadamard length, pad[1] -> clip
     RQ_CUDA(rq_configure_act());
     RQ_CUDA(rq_configure_gemm_tc());
+    RQ_CUDA(rq_configure_gemm_w4());
     rq_block hdr;
     uint8_t * pp = static_cast<uint8_t *>(prepack_dev);
     int32_t * flag_dev = reinterpret_cast<int32_t *>(pp + l.off_wk);   // scratch until the pack kernel overwrites it
@@ -317,7 +318,7 @@ static int rq_use_tc(const rq_weight_desc * w, int64_t M, int path) {
     const bool has_dec = (w->layouts & RQ_PREPACK_DECODE) != 0, has_pre = (w->layouts & RQ_PREPACK_PREFILL) != 0;
     if (path == RQ_PATH_GEMV) return has_dec ? 0 : -1;
     if (path == RQ_PATH_TC) return has_pre ? 1 : -1;
-    // up to 64 tokens the GEMV in passes of 16 (the later passes read the stream from L2) beats a 128-token MMA tile
+    // up to 64 tokens the kernels that read the int4 stream (half the bytes, one pass) beat a 128-token MMA tile
     if (path == RQ_PATH_AUTO) return (has_pre && (M > 64 || !has_dec)) ? 1 : (has_dec ? 0 : -1);
     return -1;
 }

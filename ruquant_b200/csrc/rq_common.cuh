@@ -36,6 +36,11 @@ __host__ __device__ inline int rq_wmult(int32_t sum, int g) {
 __host__ __device__ inline int rq_perm64(int k4) {   // k4: offset of a 4-input piece inside the run (multiple of 4)
     return ((k4 & 15) >> 2) * 16 + (k4 >> 4) * 4;
 }
+// Decode stream: the 16-byte slot, inside the 512 bytes of a 16-row tile's run of 64 inputs, that holds words (2*b + h),
+// b, h in 0..1, of row gid + 8*b: low nibbles inputs 32*h + 4*tig .. +3, high nibbles those 16 further.  The XOR makes both
+// readers conflict-free: the GEMV's warp (lane = 4*gid + tig reads a slot, 8 lanes a phase: two gids, four tigs) and the batch
+// kernel's (lane = row reads half a slot of one tig, 16 rows a phase).
+__host__ __device__ inline int rq_w4_slot(int gid, int tig) { return tig * 8 + (gid ^ (tig * 2)); }
 // e4m3 byte of a small integer (|v| <= 15: at most four significant bits, so the conversion is exact)
 __host__ __device__ inline uint32_t rq_e4m3_of_int(int v) {
     const uint32_t sign = v < 0 ? 0x80u : 0u;
@@ -145,6 +150,9 @@ struct rq_gemv_job {
 };
 cudaError_t rq_launch_gemv(const rq_gemv_job * jobs, int n_jobs, int64_t K, const int8_t * a8, const int32_t * msh,
                            const float * u, int64_t M, int G, int32_t * status, cudaStream_t stream);
+// the same contraction for 9 to 64 tokens at once, on the tensor cores (rq_gemm_w4.cu)
+cudaError_t rq_launch_gemm_w4(const rq_gemv_job * jobs, int n_jobs, int64_t K, const int8_t * a8, const int32_t * msh,
+                              const float * u, int64_t M, int G, int32_t * status, cudaStream_t stream);
 cudaError_t rq_launch_gemm_tc(const void * tmap_w8, const float * sw, int fmt, int64_t K, int64_t N,
                               const int8_t * a8, const int32_t * msh, const float * u, int64_t M, int G,
                               float * y, int64_t ldy, int32_t * status, cudaStream_t stream, float * const * y_more = nullptr,
@@ -164,5 +172,7 @@ cudaError_t rq_launch_wquant(const float * x, int64_t ldx, int64_t n_rows, int64
 // launch inside a stream capture has nothing left to set up
 cudaError_t rq_configure_act();
 cudaError_t rq_configure_gemm_tc();
+cudaError_t rq_configure_gemm_w4();
 // host-side: encodes the 2-D tensor map of a row-major int8 [rows][K] operand with a {128, box_rows} box, 128B swizzle
 int rq_encode_tmap_i8(void * tmap_out, const void * base, int64_t K, int64_t rows, int box_rows);
+int rq_encode_tmap_w4(void * tmap_out, const void * base, int64_t K, int64_t tiles);

@@ -815,6 +815,23 @@ int rq_encode_tmap_i8(void * tmap_out, const void * base, int64_t K, int64_t row
     return 0;
 }
 
+// the int4 decode stream as rows of 16-row tiles (K * 8 bytes each), boxes of 8 tiles x 256 inputs (2 KB), not swizzled
+int rq_encode_tmap_w4(void * tmap_out, const void * base, int64_t K, int64_t tiles) {
+    encode_fn_t fn = get_encode();
+    if (fn == nullptr) return -1;
+    alignas(64) CUtensorMap map;
+    const cuuint64_t dims[2] = { (cuuint64_t) K, (cuuint64_t) tiles };       // in 8-byte elements
+    const cuuint64_t strides[1] = { (cuuint64_t) K * 8 };
+    const cuuint32_t box[2] = { 256, 8 };
+    const cuuint32_t estr[2] = { 1, 1 };
+    const CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void *>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return -1;
+    memcpy(tmap_out, &map, sizeof(map));
+    return 0;
+}
+
 template <bool F8, bool PAIR, bool PUSH>
 static cudaError_t configure_tc() {
     return cudaFuncSetAttribute(rq_gemm_tc_kernel<F8, PAIR, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_of(PAIR));

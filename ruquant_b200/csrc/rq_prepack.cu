@@ -3,10 +3,10 @@
 // ggml/src/ggml-cuda/rq-w4a4.cu in patches/llama.cpp-ruquant.patch:1842-1880.)
 //
 //   sw  f32 [N]        the row unit s_w (block 0 of each row; every block of a row repeats it)
-//   w4  u32 [ceil(N/16) tiles][K/64 runs][32 lanes][4 words]   decode stream in consumption order: lane l = 4*gid + tig
-//                      of the GEMV warp loads its 16 bytes and unpacks word j into two int8x4 registers,
-//                      `(w << 4) & 0xF0F0F0F0` = 16*c of row tile*16 + gid and `w & 0xF0F0F0F0` = 16*c of row
-//                      tile*16 + gid + 8, inputs run*64 + (j/2)*32 + (j%2)*16 + tig*4 .. +3 -- exactly the A fragment
+//   w4  u32 [ceil(N/16) tiles][K/64 runs][32 slots][4 words]   decode stream in consumption order: lane l = 4*gid + tig
+//                      of the GEMV warp loads the 16 bytes at slot rq_w4_slot(gid, tig) and unpacks word 2*b + h into two int8x4
+//                      registers, `(w << 4) & 0xF0F0F0F0` = 16*c of row tile*16 + gid + 8*b, inputs run*64 + 32*h + 4*tig .. +3,
+//                      and `w & 0xF0F0F0F0` the same row's inputs 16 further -- exactly the A fragment
 //                      of mma.m16n8k32 (a nibble moved to the top of its byte is 16*c in two's complement: no sign
 //                      fix-up).  Rows beyond N are zero.
 //   w8  u8  [N][K]     tensor-core operand: the e4m3 byte of c when every multiplier is 1 (fp8 MMA, fp32 accumulate,
@@ -60,15 +60,15 @@ __global__ void rq_prepack_stream_kernel(const rq_block * __restrict__ blocks, i
     const int64_t ng64 = K / 64, tiles = (N + 15) / 16;
     const int64_t idx = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= tiles * ng64 * 128) return;
-    const int j = (int) (idx & 3), lane = (int) ((idx >> 2) & 31);
+    const int j = (int) (idx & 3), slot = (int) ((idx >> 2) & 31);
     const int64_t g64 = (idx >> 7) % ng64, tile = (idx >> 7) / ng64;
-    const int gid = lane >> 2, tig = lane & 3;
-    const int64_t k0 = g64 * 64 + (j >> 1) * 32 + (j & 1) * 16 + tig * 4;
+    const int tig = slot >> 3, gid = (slot & 7) ^ (tig * 2);       // the inverse of rq_w4_slot
+    const int64_t row = tile * 16 + gid + 8 * (j >> 1);
     uint32_t dst = 0;
+    if (row < N) {
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int64_t row = tile * 16 + gid + 8 * half;
-        if (row < N) {
+        for (int half = 0; half < 2; ++half) {
+            const int64_t k0 = g64 * 64 + (j & 1) * 32 + half * 16 + tig * 4;
             const rq_block * b = blocks + row * (K / RQ_BLOCK_CODES) + k0 / RQ_BLOCK_CODES;
             const uint32_t src = b->qs[(k0 % RQ_BLOCK_CODES) / 8] >> (4 * (k0 % 8));     // 4 codes from bit 0
 #pragma unroll
