@@ -56,6 +56,26 @@ def test_random_rows_match_the_oracle(rq, port, type_, wgroup):
         assert (got == want).all(), (type_, wgroup, K, N, np.argwhere(got != want)[:4])
 
 
+@pytest.mark.parametrize("wgroup", [0, 256, 64])
+@pytest.mark.parametrize("K", [256, 768, 5120, 32768])
+def test_near_ties_and_extreme_rows_match_the_oracle(rq, port, K, wgroup):
+    """Rows on which the choice of the scale is close or the fast sums do not apply: few distinct values (candidates with equal
+    errors), values on the code grid of one candidate (halves that round either way), one large value among small ones,
+    magnitudes outside the range of the fast sums, subnormals; many random rows for the near-ties that come by themselves."""
+    rng = np.random.default_rng(K + wgroup)
+    rows = [np.where(rng.random(K) < 0.5, 1.0, -1.0), np.full(K, 0.3), rng.integers(-7, 8, K) * 0.125, rng.integers(-14, 15, K) * 0.5,
+            np.concatenate([[100.0], rng.normal(0, 1e-3, K - 1)]), rng.normal(0, 1e30, K), rng.normal(0, 1e-41, K), rng.normal(0, 1e-25, K),
+            np.where(rng.random(K) < 0.01, 1e13, 1.0), rng.integers(0, 2, K) * 7.0]
+    for r in range(0, 13):          # halves of candidate r's scale for a row whose largest value is 7
+        s = np.float32(np.float32(7.0) * np.float32(np.float32(1.0) - np.float32(np.float32(0.025) * np.float32(r)))) / np.float32(7.0)
+        v = (rng.integers(-7, 7, K) + 0.5) * s
+        v[0] = 7.0
+        rows.append(v)
+    w = np.concatenate([np.stack(rows), rng.normal(0, 0.02, (200 if K <= 768 else 16, K))]).astype(np.float32)
+    want, got = port.quantize_weights(w, 44, wgroup=wgroup), gpu_blocks(rq, w, 44, wgroup)
+    assert (got == want).all(), (K, wgroup, np.unique(np.argwhere(got != want)[:, 0]))
+
+
 def test_rotation_blocks_and_strided_rows(rq, port):
     K, N = 5120, 24
     w = inputs.normal_weights(N, K + 64, 7100)[:, :K]          # rows 5184 floats apart
