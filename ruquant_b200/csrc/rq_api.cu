@@ -313,6 +313,14 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_quantize_rows(cons
     return RQ_OK;
 }
 
+static rq_gemm_job rq_tc_job(const rq_weight_desc * w, float * y, int64_t ldy) {
+    rq_gemm_job job = {};
+    const uint8_t * pp = static_cast<const uint8_t *>(w->prepack);
+    job.tmap_w8 = w->tmap_w8; job.w8 = pp + w->off_w8; job.sw = reinterpret_cast<const float *>(pp + w->off_sw);
+    job.N = w->N; job.y = y; job.ldy = ldy;
+    return job;
+}
+
 // which kernel a weight takes at M tokens: true = tcgen05 GEMM, false = GEMV passes; -1 on a bad request
 static int rq_use_tc(const rq_weight_desc * w, int64_t M, int path) {
     const bool has_dec = (w->layouts & RQ_PREPACK_DECODE) != 0, has_pre = (w->layouts & RQ_PREPACK_PREFILL) != 0;
@@ -357,7 +365,8 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_mul_mat_quantized(
     const bool tc = use_tc != 0;
     int32_t * status = reinterpret_cast<int32_t *>(const_cast<uint8_t *>(ws) + l.off_status);
     if (tc) {
-        RQ_CUDA(rq_launch_gemm_tc(w->tmap_w8, sw, w->wk_mode ? RQ_FMT_I8 : RQ_FMT_E4M3, w->K, w->N, a8, msh, u, M, act_group, y_dev, ldy, status, stream));
+        const rq_gemm_job job = rq_tc_job(w, y_dev, ldy);
+        RQ_CUDA(rq_launch_gemm_tc(&job, 1, w->wk_mode ? RQ_FMT_I8 : RQ_FMT_E4M3, w->K, a8, msh, u, M, act_group, status, stream));
     } else {
         rq_gemv_job job;
         job.w4 = pp + w->off_w4; job.sw = sw; job.N = w->N; job.y = y_dev; job.ldy = ldy; job.n_more = 0;
@@ -379,9 +388,9 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_tc_nofold_probe(co
     if (workspace_dev == nullptr || workspace_bytes < l.bytes) return RQ_ERR_WORKSPACE;
     const uint8_t * ws = static_cast<const uint8_t *>(workspace_dev);
     const uint8_t * pp = static_cast<const uint8_t *>(w->prepack);
-    RQ_CUDA(rq_launch_gemm_tc(w->tmap_w8, reinterpret_cast<const float *>(pp + w->off_sw), w->wk_mode ? RQ_FMT_I8 : RQ_FMT_E4M3, w->K, w->N,
-                              reinterpret_cast<const int8_t *>(ws + l.off_a8), reinterpret_cast<const int32_t *>(ws + l.off_msh),
-                              reinterpret_cast<const float *>(ws + l.off_u), M, (int) w->K, y_dev, ldy,
+    const rq_gemm_job job = rq_tc_job(w, y_dev, ldy);
+    RQ_CUDA(rq_launch_gemm_tc(&job, 1, w->wk_mode ? RQ_FMT_I8 : RQ_FMT_E4M3, w->K, reinterpret_cast<const int8_t *>(ws + l.off_a8),
+                              reinterpret_cast<const int32_t *>(ws + l.off_msh), reinterpret_cast<const float *>(ws + l.off_u), M, (int) w->K,
                               reinterpret_cast<int32_t *>(const_cast<uint8_t *>(ws) + l.off_status), (cudaStream_t) stream));
     return RQ_OK;
 }
@@ -419,6 +428,23 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_mul_mat_quantized_
         RQ_CUDA(rq_launch_gemv(jobs, n_w, w[0]->K, reinterpret_cast<const int8_t *>(ws + l.off_a8),
                                reinterpret_cast<const int32_t *>(ws + l.off_msh), reinterpret_cast<const float *>(ws + l.off_u), M,
                                act_group, reinterpret_cast<int32_t *>(ws + l.off_status), (cudaStream_t) stream));
+        return RQ_OK;
+    }
+    // prefill widths: likewise one launch when they all take the tcgen05 kernel in the same operand format
+    bool one_tc = n_w > 1;
+    for (int i = 0; i < n_w && one_tc; ++i) {
+        one_tc = w[i]->prepack != nullptr && rq_use_tc(w[i], M, path) == 1 && w[i]->wk_mode == w[0]->wk_mode && ldy[i] >= w[i]->N &&
+                 !(w[i]->wg64 && act_group != 64);
+    }
+    if (one_tc) {
+        const rq_ws_layout l = rq_ws(w[0]->K, M);
+        if (workspace_dev == nullptr || workspace_bytes < l.bytes) return RQ_ERR_WORKSPACE;
+        uint8_t * ws = static_cast<uint8_t *>(workspace_dev);
+        rq_gemm_job jobs[RQ_MAX_WEIGHTS];
+        for (int i = 0; i < n_w; ++i) jobs[i] = rq_tc_job(w[i], y_dev[i], ldy[i]);
+        RQ_CUDA(rq_launch_gemm_tc(jobs, n_w, w[0]->wk_mode ? RQ_FMT_I8 : RQ_FMT_E4M3, w[0]->K, reinterpret_cast<const int8_t *>(ws + l.off_a8),
+                                  reinterpret_cast<const int32_t *>(ws + l.off_msh), reinterpret_cast<const float *>(ws + l.off_u), M, act_group,
+                                  reinterpret_cast<int32_t *>(ws + l.off_status), (cudaStream_t) stream));
         return RQ_OK;
     }
     for (int i = 0; i < n_w; ++i) {
@@ -473,13 +499,12 @@ extern "C" __attribute__((visibility("default"))) int rq_w4a4_mul_mat_push(const
     uint8_t * ws = static_cast<uint8_t *>(workspace_dev);
     if (tc) {
         for (int i = 0; i < n_w; ++i) {
-            const uint8_t * pp = static_cast<const uint8_t *>(w[i]->prepack);
-            float * more[RQ_MAX_RANKS - 1];
-            for (int d = 1; d < n_dst; ++d) more[d - 1] = y_dst[d * n_w + i];
-            RQ_CUDA(rq_launch_gemm_tc(w[i]->tmap_w8, reinterpret_cast<const float *>(pp + w[i]->off_sw), fmt, w[i]->K, w[i]->N,
-                                      reinterpret_cast<const int8_t *>(ws + l.off_a8), reinterpret_cast<const int32_t *>(ws + l.off_msh),
-                                      reinterpret_cast<const float *>(ws + l.off_u), M, act_group, y_dst[i], ldy[i],
-                                      reinterpret_cast<int32_t *>(ws + l.off_status), (cudaStream_t) stream, more, n_dst - 1));
+            rq_gemm_job job = rq_tc_job(w[i], y_dst[i], ldy[i]);
+            job.n_more = n_dst - 1;
+            for (int d = 1; d < n_dst; ++d) job.y_more[d - 1] = y_dst[d * n_w + i];
+            RQ_CUDA(rq_launch_gemm_tc(&job, 1, fmt, w[i]->K, reinterpret_cast<const int8_t *>(ws + l.off_a8),
+                                      reinterpret_cast<const int32_t *>(ws + l.off_msh), reinterpret_cast<const float *>(ws + l.off_u), M, act_group,
+                                      reinterpret_cast<int32_t *>(ws + l.off_status), (cudaStream_t) stream));
         }
         return RQ_OK;
     }

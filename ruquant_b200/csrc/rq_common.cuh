@@ -153,10 +153,19 @@ cudaError_t rq_launch_gemv(const rq_gemv_job * jobs, int n_jobs, int64_t K, cons
 // the same contraction for 9 to 64 tokens at once, on the tensor cores (rq_gemm_w4.cu)
 cudaError_t rq_launch_gemm_w4(const rq_gemv_job * jobs, int n_jobs, int64_t K, const int8_t * a8, const int32_t * msh,
                               const float * u, int64_t M, int G, int32_t * status, cudaStream_t stream);
-cudaError_t rq_launch_gemm_tc(const void * tmap_w8, const float * sw, int fmt, int64_t K, int64_t N,
-                              const int8_t * a8, const int32_t * msh, const float * u, int64_t M, int G,
-                              float * y, int64_t ldy, int32_t * status, cudaStream_t stream, float * const * y_more = nullptr,
-                              int n_more = 0);
+// one weight of a prefill launch; all jobs of a launch share K, the activation and its format, and only a single one may push
+struct rq_gemm_job {
+    const void * tmap_w8;  // boxes of 128 inputs x 128 rows
+    const uint8_t * w8;
+    const float * sw;
+    int64_t N;
+    float * y;
+    int64_t ldy;
+    float * y_more[RQ_MAX_RANKS - 1];
+    int n_more;
+};
+cudaError_t rq_launch_gemm_tc(const rq_gemm_job * jobs, int n_jobs, int fmt, int64_t K, const int8_t * a8, const int32_t * msh, const float * u,
+                              int64_t M, int G, int32_t * status, cudaStream_t stream);
 // all-ranks barrier over peer-mapped flag words (rq_rank.cu)
 cudaError_t rq_launch_rank_barrier(uint32_t * const * flags_of_rank, int rank, int n_ranks, uint32_t * epoch, int32_t * status,
                                    cudaStream_t stream);
