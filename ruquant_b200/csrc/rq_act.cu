@@ -12,8 +12,12 @@
 // (q - z_g) and the f32 bits of m_g / 16.
 //
 // Two kernels:
-//   rq_act_kernel<P>          one CTA per token, the token's row resident in shared memory (prefill widths, any G).
-//   rq_act_cluster_kernel<P>  a thread-block cluster per token for decode widths: every CTA transforms the whole row
+//   rq_act_kernel<P>          one CTA per token, the token's row resident in shared memory (prefill widths, any G).  What bounds it
+//                             at thousands of tokens: the Paley adds (K = 17408: 134 of 268 us for 4096 tokens, the rate of the
+//                             fp32 pipe, as packed adds with the signs in the code; 294 before), the rest is load 33, Sylvester 48,
+//                             quantizer 53 us -- phases of one CTA that overlap only with those of the SM's two others.
+//                             K = 5120: 49 us, 68 before.
+//   rq_act_cluster_kernel<P>  a thread-block cluster per token for decode and batch widths: every CTA transforms the whole row
 //                             (redundant, but it spares a gather through distributed shared memory), the Paley outputs
 //                             are split between the CTAs, and one cluster barrier agrees on the token's range.
 // Both start their successor early (programmatic dependent launch) and build the sign table before they wait for
@@ -32,7 +36,10 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int ACT_THREADS = 256;
+// threads of a prefill CTA: Paley orders up to 72 take two columns per thread (all of them in registers), larger ones one
+constexpr int act_threads(int p) { return p > 1 && p <= 72 ? 128 : 256; }
+constexpr bool act_both(int p) { return p > 44 && p <= 72; }         // 256 threads and a column each where few tokens leave SMs short of warps
+constexpr int act_min_ctas(int p) { return p <= 1 || p > 72 ? 3 : p <= 20 ? 6 : p <= 44 ? 4 : 3; }
 // threads of a cluster CTA: every phase is latency, so as many warps as the Paley stage's registers allow (it reads its
 // P inputs once each, the compiler keeps them at about 55-64 registers)
 constexpr int cluster_threads(int p) { return p <= 72 ? 1024 : 512; }
@@ -56,12 +63,8 @@ struct ActParams {
 // =====================================================================================  one CTA per token
 // P > 1: Paley order (compile time); P == 1: no Paley stage (plain W4A4, or a power-of-two rotation).
 // shared memory: [K floats row][P*P floats sign table]
-// three CTAs (tokens) per SM where the row fits three times in shared memory: caps the 256-thread form at 85 registers
-#ifndef RQ_ACT_MIN_CTAS
-#define RQ_ACT_MIN_CTAS 3
-#endif
 template <int P, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? RQ_ACT_MIN_CTAS : 1) rq_act_kernel(const ActParams prm) {
+__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P) : 1) rq_act_kernel(const ActParams prm) {
     extern __shared__ __align__(16) float buf[];
     __shared__ float g_lo[512], g_hi[512];
     __shared__ float red[THREADS / 32];
@@ -100,6 +103,15 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? RQ_ACT_MIN_CTAS : 1)
         const int m = prm.m;
         if constexpr (P > 1) {
             const int ncol = K / P, n = prm.n_rot;
+            if constexpr (THREADS == 128) {
+                if (m > 1) {
+                    for (int c = 2 * tid; c < ncol; c += 2 * nt) {
+                        const int blk = c / m, j = c - blk * m;
+                        paley_pair<P>(buf + (size_t) blk * n + j, m, prm.rot_scale);
+                    }
+                }
+            }
+            if (THREADS != 128 || m == 1) {
             if constexpr (P <= 20 && THREADS <= 256) {
                 // many tokens in flight (one CTA each): the adds themselves are the work, signs folded into the code
                 for (int c = tid; c < ncol; c += nt) {
@@ -131,6 +143,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? RQ_ACT_MIN_CTAS : 1)
                     for (int k = 0; k < 4; ++k) b[(a0 + k) * m] = out[k];
                 }
             }
+            }
         } else {
             for (int i = tid; i < K; i += nt) buf[i] = __fmul_rn(buf[i], prm.rot_scale);
         }
@@ -143,13 +156,15 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? RQ_ACT_MIN_CTAS : 1)
     if (prm.a8 == nullptr) return;
     RQ_STAMP(tid == 0);                                     // 3: Paley done
 
-    // ---- quantizer: a thread owns a word of 8 values, G/8 neighbouring lanes own a group
+    // ---- quantizer: 8 lanes own a run of 64 values, G/8 neighbouring lanes a group
     const int lpg = prm.G >> 3, nwords = K >> 3;
-    const int llpg = __ffs(lpg) - 1;                        // G / 8 is a power of two: a shift, not a division, per word
+    const int llpg = __ffs(lpg) - 1;                        // G / 8 is a power of two: a shift, not a division, per lane
+    const int l = tid & 7, off_a = run_piece(l, 0), off_b = run_piece(l, 1);
+    const float4 * buf4 = reinterpret_cast<const float4 *>(buf);
     float tmax = 0.0f;
     for (int w = tid; w < nwords; w += nt) {
         float lo, hi;
-        group_range(reinterpret_cast<float4 *>(buf)[2 * w], reinterpret_cast<float4 *>(buf)[2 * w + 1], lpg, prm.clip, lo, hi);
+        group_range(buf4[(w >> 3) * 16 + off_a], buf4[(w >> 3) * 16 + off_b], lpg, prm.clip, lo, hi);
         if ((w & (lpg - 1)) == 0) {
             g_lo[w >> llpg] = lo;
             g_hi[w >> llpg] = hi;
@@ -165,19 +180,23 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? RQ_ACT_MIN_CTAS : 1)
     if (tid == 0) prm.u[t] = unit;
     RQ_STAMP(tid == 0);                                     // 4: ranges reduced
 
-    int8_t * arow = prm.a8 + (int64_t) t * K;
+    // the groups' constants once per group (two divisions), in place of their ranges
     int32_t * mrow = prm.msh + (int64_t) t * (K / prm.G);
+    for (int g = tid; g < K / prm.G; g += nt) {
+        float mf, inv, zf;
+        group_constants(g_lo[g], g_hi[g], R, unit, mf, inv, zf);
+        mrow[g] = prm.fmt == RQ_FMT_E4M3 ? multiplier_word<true>(mf) : multiplier_word<false>(mf);
+        g_lo[g] = inv;
+        g_hi[g] = zf;
+    }
+    __syncthreads();
+    int8_t * arow = prm.a8 + (int64_t) t * K + run_offset(l);
     auto store_codes = [&](auto f8) {
         constexpr bool F8 = decltype(f8)::value;
         for (int w = tid; w < nwords; w += nt) {
-            const int g = w >> llpg;
-            float mi;
-            const uint2 pk = encode_word<F8>(reinterpret_cast<float4 *>(buf)[2 * w], reinterpret_cast<float4 *>(buf)[2 * w + 1],
-                                             g_lo[g], g_hi[g], R, unit, mi);
-            const int kw = w * 8, run = kw & ~63, off = kw & 63;   // two 4-input pieces, permuted inside their run of 64
-            *reinterpret_cast<uint32_t *>(arow + run + rq_perm64(off)) = pk.x;
-            *reinterpret_cast<uint32_t *>(arow + run + rq_perm64(off + 4)) = pk.y;
-            if ((w & (lpg - 1)) == 0) mrow[g] = multiplier_word<F8>(mi);
+            const float inv = g_lo[w >> llpg], zf = g_hi[w >> llpg];
+            const uint32_t ca = encode4<F8>(buf4[(w >> 3) * 16 + off_a], inv, zf), cb = encode4<F8>(buf4[(w >> 3) * 16 + off_b], inv, zf);
+            *reinterpret_cast<uint2 *>(arow + (w >> 3) * 64) = run_codes(l, ca, cb);
         }
     };
     if (prm.fmt == RQ_FMT_E4M3) store_codes(std::true_type{});
@@ -245,11 +264,12 @@ __global__ void __launch_bounds__(THREADS) rq_act_cluster_kernel(const ActParams
 
     // ---- group ranges: a row of 64 outputs is one activation group (8 lanes x 8 values); nl * 32 words, so a warp is
     // inside or outside the loop as a whole
-    const int words = nl * 32;
+    const int words = nl * 32, l8 = tid & 7, off_a = run_piece(l8, 0), off_b = run_piece(l8, 1);
+    const float4 * outs4 = reinterpret_cast<const float4 *>(outs);
     float tmax = 0.0f;
     for (int w = tid; w < words; w += nt) {
         float lo, hi;
-        group_range(reinterpret_cast<float4 *>(outs)[2 * w], reinterpret_cast<float4 *>(outs)[2 * w + 1], 8, prm.clip, lo, hi);
+        group_range(outs4[(w >> 3) * 16 + off_a], outs4[(w >> 3) * 16 + off_b], 8, prm.clip, lo, hi);
         tmax = fmaxf(tmax, __fsub_rn(hi, lo));
     }
     tmax = cta_max_warp0(tmax, red, tid, nt);
@@ -273,15 +293,12 @@ __global__ void __launch_bounds__(THREADS) rq_act_cluster_kernel(const ActParams
             const int v = rank + l * C;
             const int ab = v % NB, sl = v / NB, js = sl & (nq - 1), blk = sl >> lq;
             const int kbase = blk * n + (ab * 4 + k) * m + js * 64;         // first input of this group in the row
-            const float4 a = reinterpret_cast<float4 *>(outs)[2 * w], b = reinterpret_cast<float4 *>(outs)[2 * w + 1];
-            float lo, hi;
+            const float4 a = outs4[r * 16 + off_a], b = outs4[r * 16 + off_b];
+            float lo, hi, mf, inv, zf;
             group_range(a, b, 8, prm.clip, lo, hi);
-            float mi;
-            const uint2 pk = encode_word<F8>(a, b, lo, hi, R, unit, mi);
-            const int off = (w & 7) * 8;
-            *reinterpret_cast<uint32_t *>(arow + kbase + rq_perm64(off)) = pk.x;
-            *reinterpret_cast<uint32_t *>(arow + kbase + rq_perm64(off + 4)) = pk.y;
-            if ((w & 7) == 0) mrow[kbase >> 6] = multiplier_word<F8>(mi);
+            group_constants(lo, hi, R, unit, mf, inv, zf);
+            *reinterpret_cast<uint2 *>(arow + kbase + run_offset(l8)) = run_codes(l8, encode4<F8>(a, inv, zf), encode4<F8>(b, inv, zf));
+            if (l8 == 0) mrow[kbase >> 6] = multiplier_word<F8>(mf);
         }
     };
     if (prm.fmt == RQ_FMT_E4M3) store_codes(std::true_type{});
@@ -324,14 +341,32 @@ cudaError_t configure_kernel(Kern kern) {
 
 template <int P>
 cudaError_t configure() {
-    cudaError_t e = configure_kernel(rq_act_kernel<P, ACT_THREADS>);
+    cudaError_t e = configure_kernel(rq_act_kernel<P, act_threads(P)>);
     if (e != cudaSuccess) return e;
     if (P <= 20) {
         e = configure_kernel(rq_act_kernel<(P <= 20 ? P : 1), 1024>);
         if (e != cudaSuccess) return e;
     }
+    if (act_both(P) && (e = configure_kernel(rq_act_kernel<(act_both(P) ? P : 1), 256>)) != cudaSuccess) return e;
     if (P == 1) return e;
     return configure_kernel(rq_act_cluster_kernel<(P > 1 ? P : 12), cluster_threads(P > 1 ? P : 12)>);
+}
+
+// clusters of c CTAs that run at the same time (for rows of any length: the registers allow one CTA of 1024 threads an SM)
+template <int P>
+cudaError_t clusters_at_once(int c, int * n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned) c, 148);
+    cfg.blockDim = dim3(cluster_threads(P));
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned) c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(n, rq_act_cluster_kernel<P, cluster_threads(P)>, &cfg);
 }
 
 template <int P>
@@ -339,6 +374,8 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
     // first use on a device (normally rq_w4a4_prepare's); several host threads may get here at once
     static std::mutex mu;
     static bool configured[64] = {};
+    static int sms[64] = {};
+    static int at_once[64][17] = {};       // clusters of 2, 4 and 8 CTAs that run at once
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -348,18 +385,22 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
         if (!configured[dev]) {
             e = configure<P>();
             if (e != cudaSuccess) return e;
+            if (P > 1) for (int c = 2; c <= 8; c *= 2) if ((e = clusters_at_once<(P > 1 ? P : 12)>(c, &at_once[dev][c])) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
             configured[dev] = true;
         }
     }
     const int K = prm.K;
     static const int min_p = rq_env_int("RQ_TUNE_ACT_MINP", 0);
-    if (P > 1 && P >= min_p && prm.a8 != nullptr && prm.rot_out == nullptr && prm.G == 64 && prm.m % 64 == 0 && M <= 32) {
-        // decode widths: a cluster per token
+    if (P > 1 && P >= min_p && prm.a8 != nullptr && prm.rot_out == nullptr && prm.G == 64 && prm.m % 64 == 0 && M <= at_once[dev][2]) {
+        // decode and batch widths: a cluster per token
         constexpr int CP = P > 1 ? P : 12, CT = cluster_threads(CP);
         const int units = (K / prm.n_rot) * (prm.m / 64) * (CP / 4);
+        // the widest cluster of which all M run at once: a second round costs more than the narrower cluster (16 tokens of 17408:
+        // 17.1 us with 8 CTAs a token, 10.3 with 4; 5120: 8.0 and 4.4; 64 tokens of 17408 with 2: 15.6, one CTA a token: 16.7)
         static const int c_max = rq_env_int("RQ_TUNE_ACT_CMAX", 8);
         int C = c_max;
-        while (C > 1 && units < 2 * C) C >>= 1;
+        while (C > 1 && (units < 2 * C || M > at_once[dev][C])) C >>= 1;
         const int units_max = (units + C - 1) / C;
         const size_t smem = ((size_t) K + (size_t) CP * CP + (size_t) units_max * 4 * 64) * sizeof(float);
         if (C > 1 && smem <= SMEM_LIMIT) {
@@ -372,7 +413,9 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
     // few tokens and a cheap Paley stage: one big CTA per token keeps every phase short
     static const int wide = rq_env_int("RQ_TUNE_ACT_WIDE", 1);
     if (P <= 20 && M <= 64 && wide) return launch_ex(rq_act_kernel<(P <= 20 ? P : 1), 1024>, dim3((unsigned) M), dim3(1024), smem, 1, stream, prm);
-    return launch_ex(rq_act_kernel<P, ACT_THREADS>, dim3((unsigned) M), dim3(ACT_THREADS), smem_row, 1, stream, prm);
+    // up to four tokens an SM the phases are latency: twice the warps (512 tokens of 17408: 47 us, 51 with 128 threads; 4096: 277, 268)
+    if (act_both(P) && M <= 4 * sms[dev]) return launch_ex(rq_act_kernel<(act_both(P) ? P : 1), 256>, dim3((unsigned) M), dim3(256), smem_row, 1, stream, prm);
+    return launch_ex(rq_act_kernel<P, act_threads(P)>, dim3((unsigned) M), dim3(act_threads(P)), smem_row, 1, stream, prm);
 }
 
 }  // namespace

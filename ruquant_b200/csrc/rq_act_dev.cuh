@@ -73,6 +73,48 @@ struct PaleyExt {
 };
 template <int P> __constant__ PaleyExt<P> c_paley_ext = PaleyExt<P>();
 
+// packed pairs of floats: one instruction for two columns
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float & lo, float & hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) { uint64_t r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+// All P outputs of two neighbouring columns (m even: 8-byte aligned), in place: the columns in registers, the signs in the
+// code, a packed add or subtract per two terms.  Ascending i per output, from 0.0f, as the reference sums.
+template <int P>
+__device__ __forceinline__ void paley_pair(float * b, int m, float scale) {
+    constexpr PaleyExt<P> e{};
+    uint64_t col[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) col[i] = *reinterpret_cast<const uint64_t *>(b + i * m);
+    const uint64_t scale2 = pack2(scale, scale);
+    // (the store addresses are counted up from here: derived from the loads' they would be kept in P registers)
+    asm volatile("" : "+l"(b), "+r"(m));
+#pragma unroll
+    for (int a0 = 0; a0 < P; a0 += 4) {
+        uint64_t acc[4] = { 0, 0, 0, 0 };
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int a = a0 + k;
+                const bool plus = i == a || i == 0 || (a != 0 && e.v[a - i + P - 2] > 0.0f);
+                acc[k] = plus ? add2(acc[k], col[i]) : sub2(acc[k], col[i]);
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            *reinterpret_cast<uint64_t *>(b) = mul2(acc[k], scale2);
+            b += m;
+        }
+        asm volatile("" ::: "memory");
+    }
+}
+
 // outputs a0 .. a0+3 (a0 >= 1, warp-uniform) of one column held in registers, signs from the constant table
 template <int P>
 __device__ __forceinline__ void paley_block4_const(const float (&col)[P], int a0, float scale, float (&out)[4]) {
@@ -166,8 +208,9 @@ __device__ __forceinline__ void fwht_chunks(float * buf, int len, int m, int tid
 
 // Sylvester transform of 32*EPT consecutive values held by one warp, lane l owning values [l*EPT, (l+1)*EPT): the
 // strides below EPT are butterflies between a lane's own registers, the strides EPT .. 16*EPT are exchanges with lane
-// l ^ d (the lower lane forms a + b, the upper lane a - b with a the lower lane's value) -- the same operations in the
-// same order as the reference's loop, without touching shared memory.
+// l ^ d (the lower lane forms a + b, the upper lane a - b with a the lower lane's value; as a fused multiply-add by +-1 the
+// product is exact and the rounding the same) -- the same operations in the same order as the reference's loop, without
+// touching shared memory.
 template <int EPT>
 __device__ __forceinline__ void fwht_warp(float (&v)[EPT], int lane) {
 #pragma unroll
@@ -183,12 +226,9 @@ __device__ __forceinline__ void fwht_warp(float (&v)[EPT], int lane) {
     }
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const bool upper = (lane & d) != 0;
+        const float sign = (lane & d) != 0 ? -1.0f : 1.0f;
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[j], d);
-            v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
-        }
+        for (int j = 0; j < EPT; ++j) v[j] = __fmaf_rn(v[j], sign, __shfl_xor_sync(0xffffffffu, v[j], d));
     }
 }
 
@@ -251,7 +291,10 @@ __device__ __forceinline__ void transform_runs_inplace(float * buf, int count, i
 // Sylvester transform, chunk by chunk, of a row that is already in shared memory.  Ends with a CTA barrier.
 __device__ __forceinline__ void fwht_resident(float * buf, int len, int m, int tid, int nt, int bar = 0) {
     const int warp = tid >> 5, nwarps = nt >> 5, lane = tid & 31;
-    const int run = m < 1024 ? m : 1024;
+    // register runs of up to 1024 values, shorter (down to 256) where there would be fewer of them than warps (4096 tokens of
+    // 4096: 85 us with the four runs of 1024 on eight warps, 65 with 16 of 256 and two passes over shared memory)
+    int run = m < 1024 ? m : 1024;
+    while (run > 256 && len / run < nwarps) run >>= 1;
     switch (run) {
         case 32:   if (m > 1) transform_runs_inplace<1>(buf, len / 32, warp, nwarps, lane); break;
         case 64:   transform_runs_inplace<2>(buf, len / 64, warp, nwarps, lane); break;
@@ -262,7 +305,7 @@ __device__ __forceinline__ void fwht_resident(float * buf, int len, int m, int t
         default:   fwht_chunks(buf, len, m, tid, nt, bar); return;      // m < 32: the generic passes
     }
     rq_cta_sync(bar, nt);
-    for (int ls = 10; (1 << ls) < m; ls += 3) {
+    for (int ls = __ffs(run) - 1; (1 << ls) < m; ls += 3) {
         const int rem = m >> ls;
         if (rem >= 8) fwht_pass<8>(buf, len, ls, tid, nt);
         else if (rem == 4) fwht_pass<4>(buf, len, ls, tid, nt);
@@ -323,7 +366,7 @@ __device__ __forceinline__ void load_fwht(const float * __restrict__ src, float 
 
 // ---- quantizer pieces shared by both kernels
 
-// range of a word of 8 values reduced over the lpg lanes that share its group
+// range of 8 values reduced over the lpg lanes that share their group
 __device__ __forceinline__ void group_range(const float4 a, const float4 b, int lpg, float clip, float & lo, float & hi) {
     float mn = fminf(fminf(fminf(a.x, a.y), fminf(a.z, a.w)), fminf(fminf(b.x, b.y), fminf(b.z, b.w)));
     float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
@@ -337,52 +380,61 @@ __device__ __forceinline__ void group_range(const float4 a, const float4 b, int 
     hi = __fmul_rn(mx, clip);
 }
 
-// the 8 codes of a word and the group's multiplier.  F8 false: int8 8*(q - z) (RQ_FMT_I8); true: the e4m3 byte of
+constexpr float ACT_MAGIC = 12582912.0f;       // 1.5 * 2^23
+
+// multiplier, 1 / scale and zero point of a group
+__device__ __forceinline__ void group_constants(float lo, float hi, float R, float unit, float & mf, float & inv, float & zf) {
+    mf = fminf(fmaxf(ceilf(__fdiv_rn(__fmul_rn(__fsub_rn(hi, lo), 255.0f), R)), 1.0f), 255.0f);
+    inv = __fdiv_rn(1.0f, __fmul_rn(mf, unit));
+    zf = fminf(fmaxf(__fsub_rn(__fadd_rn(__fmul_rn(-lo, inv), ACT_MAGIC), ACT_MAGIC), 0.0f), 15.0f);
+}
+
+// the codes of 4 values, one byte each.  F8 false: int8 8*(q - z) (RQ_FMT_I8); true: the e4m3 byte of
 // (q - z), exact (RQ_FMT_E4M3, the fp8 tensor-core path).  Everything stays in float registers: conversions between
-// float and int run at a quarter of the FMA rate on this part and integer logic at half of it, and this loop runs once
+// float and int run at a quarter of the FMA rate on this part and integer logic at half of it, and this runs once
 // per input value.
-//   rint(t)        (t + 1.5*2^23) - 1.5*2^23: round-to-nearest-even of the add, exact for |t| < 2^22; beyond that the
-//                  result may be off by one, at magnitudes the clamp to [0, 15] that follows maps to the same end
+//   rint(t)        t + 1.5*2^23, round-to-nearest-even of the add, exact for |t| < 2^22; beyond that the
+//                  result may be off by one, at magnitudes the clamp that follows maps to the same end
+//   q - z          clamp(rint(t) + z, 0, 15) - z = clamp(rint(t), -z, 15 - z), taken before the 1.5*2^23 goes off again
+//                  (all integers below 2^24: exact); a NaN ends at -z either way
 //   byte, int8     the low mantissa byte of 8*(q - z) + 1.5*2^23 is the value's two's-complement byte
 //   byte, e4m3     cvt.rn.satfinite.e4m3x2.f32 on two values at once (|q - z| <= 15 has four significant bits: exact)
 template <bool F8>
-__device__ __forceinline__ uint2 encode_word(const float4 a, const float4 b, float lo, float hi, float R, float unit, float & mf_out) {
-    const float mf = fminf(fmaxf(ceilf(__fdiv_rn(__fmul_rn(__fsub_rn(hi, lo), 255.0f), R)), 1.0f), 255.0f);
-    mf_out = mf;
-    const float inv = __fdiv_rn(1.0f, __fmul_rn(mf, unit));
-    constexpr float MAGIC = 12582912.0f;
-    const float zf = fminf(fmaxf(__fsub_rn(__fadd_rn(__fmul_rn(-lo, inv), MAGIC), MAGIC), 0.0f), 15.0f);
-    const float v[8] = { a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w };
-    float dz[8];
+__device__ __forceinline__ uint32_t encode4(const float4 a, float inv, float zf) {
+    const float lo = __fsub_rn(ACT_MAGIC, zf), hi = __fadd_rn(lo, 15.0f);
+    const uint64_t magic2 = pack2(ACT_MAGIC, ACT_MAGIC), unmagic2 = pack2(-ACT_MAGIC, -ACT_MAGIC);
+    const float v[4] = { a.x, a.y, a.z, a.w };
+    float dz[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const float r = __fsub_rn(__fadd_rn(__fmul_rn(v[j], inv), MAGIC), MAGIC);
-        const float qf = fminf(fmaxf(__fadd_rn(r, zf), 0.0f), 15.0f);
-        dz[j] = __fsub_rn(qf, zf);                                           // q - z in [-15, 15]
+    for (int h = 0; h < 2; ++h) {
+        float t0, t1;
+        // (scalar products: a packed multiply and add are contracted into one rounding, whatever -fmad says)
+        unpack2(add2(pack2(__fmul_rn(v[2 * h], inv), __fmul_rn(v[2 * h + 1], inv)), magic2), t0, t1);
+        unpack2(add2(pack2(fminf(fmaxf(t0, lo), hi), fminf(fmaxf(t1, lo), hi)), unmagic2), dz[2 * h], dz[2 * h + 1]);
     }
-    uint32_t pk[2];
     if constexpr (F8) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint16_t p01, p23;      // the second source operand lands in the low byte
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(p01) : "f"(dz[4 * h + 1]), "f"(dz[4 * h]));
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(p23) : "f"(dz[4 * h + 3]), "f"(dz[4 * h + 2]));
-            pk[h] = (uint32_t) p01 | ((uint32_t) p23 << 16);
-        }
+        uint16_t p01, p23;      // the second source operand lands in the low byte
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(p01) : "f"(dz[1]), "f"(dz[0]));
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(p23) : "f"(dz[3]), "f"(dz[2]));
+        return (uint32_t) p01 | ((uint32_t) p23 << 16);
     } else {
+        uint32_t w[4], lo01, lo23, r;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = __float_as_uint(__fmaf_rn(dz[4 * h + j], (float) RQ_ACT_SCALE, MAGIC));
-            uint32_t lo01, lo23;
-            asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(lo01) : "r"(w[0]), "r"(w[1]));      // {w0.b0, w1.b0, ., .}
-            asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(lo23) : "r"(w[2]), "r"(w[3]));
-            asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(pk[h]) : "r"(lo01), "r"(lo23));     // {lo01.b0, lo01.b1, lo23.b0, lo23.b1}
-        }
+        for (int j = 0; j < 4; ++j) w[j] = __float_as_uint(__fmaf_rn(dz[j], (float) RQ_ACT_SCALE, ACT_MAGIC));
+        asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(lo01) : "r"(w[0]), "r"(w[1]));      // {w0.b0, w1.b0, ., .}
+        asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(lo23) : "r"(w[2]), "r"(w[3]));
+        asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(r) : "r"(lo01), "r"(lo23));         // {lo01.b0, lo01.b1, lo23.b0, lo23.b1}
+        return r;
     }
-    return make_uint2(pk[0], pk[1]);
 }
+// A run of 64 values (16 pieces of 4) is held by 8 lanes, two pieces each: lane l takes pieces p = (l & 3) + 8 * (l >> 2) and
+// p + 4, which are neighbours in the permuted order of the codes (rq_perm64), so that it stores 8 bytes at byte run_offset(l);
+// the upper four lanes read their pieces in the other order, which keeps 8 lanes' 16-byte reads on different banks.
+__device__ __forceinline__ int run_piece(int l, int second) { return (l & 3) + (l & 4) * 2 + (((l >> 2) ^ second) & 1) * 4; }
+__device__ __forceinline__ int run_offset(int l) { return (l & 3) * 16 + (l & 4) * 2; }
+// the 8 bytes of a lane from the codes of its first- and second-read piece
+__device__ __forceinline__ uint2 run_codes(int l, uint32_t first, uint32_t second) { return l & 4 ? make_uint2(second, first) : make_uint2(first, second); }
+
 // what the multiplier word holds: m_g as an integer, or for the fp8 path the f32 bits of m_g / 16 (exact)
 template <bool F8>
 __device__ __forceinline__ int multiplier_word(float mf) {
