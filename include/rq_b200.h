@@ -186,7 +186,7 @@ int rq_w4a4_workspace_layout(int64_t K, int64_t M, int act_group, uint64_t * off
 int rq_w4a4_device_status(void * workspace_dev, int64_t K, int64_t M, void * stream);
 
 /* N-sharded ranks of one node (the reference assembles the outputs with a collective after the node; here the node
- * writes them itself).  rq_w4a4_mul_mat_push is rq_w4a4_mul_mat (GEMV up to 64 tokens: needs the decode layout; tcgen05
+ * writes them itself).  rq_w4a4_mul_mat_push is rq_w4a4_mul_mat (int4 stream up to 64 tokens: needs the decode layout; tcgen05
  * kernel above: needs the prefill layout) that leaves every output value in n_dst buffers instead of one (the GEMV's epilogue
  * stores it into each; in the tcgen05 kernel two warps copy every finished unit from the first buffer into the others while
  * the next units are computed): y_dst[d * n_w + i] is weight i's output in destination d
