@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "rq_common.cuh"
+#include "rq_gemm_w4_plan.h"
 
 namespace {
 
@@ -48,16 +49,11 @@ constexpr uint32_t W_BYTES = ROWS * SLICE / 2;  // 16 KB of codes per stage
 constexpr uint32_t SUB_BYTES = W_BYTES / 8;     // the part of one 16-row tile of the decode stream (a row of the TMA box)
 constexpr int THREADS = 640;
 constexpr int UNPACK_WARPS = 8;
-constexpr int MS = 4;                           // stages of the multiplier ring
-constexpr uint32_t TMEM_COLS = 512;
+constexpr int MS = RQ_W4_M_STAGES;
+constexpr uint32_t TMEM_COLS = RQ_W4_TMEM_COLS;
 constexpr int MAX_SPLIT = 8;
 constexpr long long WAIT_CYCLES = 2000000000ll;
 
-// runs of a step, A buffers of a step each, accumulator sets of a step each (SR * nt columns)
-__host__ __device__ constexpr int sr_of(int nt) { return nt <= 32 ? 4 : 2; }
-__host__ __device__ constexpr int na_of(int nt) { return 4; }
-__host__ __device__ constexpr uint32_t d_col_of(int nt) { return (uint32_t) (na_of(nt) * sr_of(nt) * 16); }
-__host__ __device__ constexpr int nd_of(int nt) { return (int) (TMEM_COLS - d_col_of(nt)) / (sr_of(nt) * nt); }
 constexpr int MAX_BUFS = 8, MAX_STAGES = 9;
 // Two rings: a weight slot is free as soon as it is unpacked, an activation slot when the MMAs have read it, steps later (in one
 // ring the weights would hold their slots as long: at 16 tokens half of the ring was not in flight)
@@ -215,7 +211,9 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                   const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2, const W4Params prm) {
     constexpr int W_STAGES = w_stages_of(NT), B_STAGES = b_stages_of(NT);
     constexpr int CG = NT <= 16 ? 4 : NT <= 32 ? 2 : 1;      // groups a fold warp takes at a time (up to 64 sums)
-    constexpr int SR = sr_of(NT), NA = na_of(NT), ND = nd_of(NT);
+    constexpr int SR = rq_w4_sr(NT), NA = rq_w4_na(NT), ND = rq_w4_nd(NT), NF = rq_w4_full_bars(NT);
+    static_assert(NA <= MAX_BUFS && ND <= MAX_BUFS && NF <= MAX_BUFS, "barriers");
+    static_assert(NF % RQ_W4_FOLD_TEAMS == 0 && MS % RQ_W4_FOLD_TEAMS == 0, "a fold warp meets every phase of a barrier that it waits on");
     extern __shared__ uint8_t smem_raw[];
     __shared__ W4Shared sh;
     const uint32_t raw = smem_u32(smem_raw), ring = (raw + 1023u) & ~1023u;
@@ -229,7 +227,7 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int tiles = prm.tile_start[prm.n_jobs], first = (int) blockIdx.x / split, stride = (int) gridDim.x / split;
     const int nsl = K / SLICE, sl0 = nsl * rank / split, sl1 = nsl * (rank + 1) / split, n_sl = sl1 - sl0;
     const int gsteps = prm.G >> 6, gps = RUNS / gsteps;       // runs per activation group, groups per slice
-    const int dgroups = SR >= gsteps ? SR / gsteps : 1, dsets = gps / dgroups;      // groups of an accumulator set, sets per slice
+    const int dgroups = rq_w4_set_groups(NT, gsteps), dsets = gps / dgroups;      // groups of an accumulator set, sets per slice
     volatile int * abort_flag = &sh.abort_flag;
 
     if (threadIdx.x == 0) rq_trace(prm.status, 0x5c);
@@ -237,7 +235,8 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int s = 0; s < W_STAGES; ++s) { mbar_init(smem_u32(&sh.full_w[s]), 1); mbar_init(smem_u32(&sh.empty_w[s]), UNPACK_WARPS); }
         for (int s = 0; s < B_STAGES; ++s) { mbar_init(smem_u32(&sh.full_b[s]), 1); mbar_init(smem_u32(&sh.empty_b[s]), 1); }
         for (int b = 0; b < NA; ++b) { mbar_init(smem_u32(&sh.a_full[b]), UNPACK_WARPS); mbar_init(smem_u32(&sh.a_empty[b]), 1); }
-        for (int b = 0; b < ND; ++b) { mbar_init(smem_u32(&sh.d_full[b]), 1); mbar_init(smem_u32(&sh.d_empty[b]), 4); }
+        for (int b = 0; b < ND; ++b) mbar_init(smem_u32(&sh.d_empty[b]), 4);
+        for (int b = 0; b < NF; ++b) mbar_init(smem_u32(&sh.d_full[b]), 1);
         for (int b = 0; b < MS; ++b) { mbar_init(smem_u32(&sh.m_full[b]), 1); mbar_init(smem_u32(&sh.m_empty[b]), 4 * dsets); }
         sh.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -351,7 +350,8 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             constexpr int GS = decltype(gsc)::value;
             uint32_t s = 0, ph = 0;               // ring slot and its phase
             uint32_t ab = 0, aph = 0;             // A buffer
-            uint32_t db = 0, dph = 1;             // accumulator set
+            uint32_t db = 0, dph = 1;             // accumulator buffer
+            uint32_t fb = 0;                      // barrier its set completes on
             const uint64_t db0 = umma_desc(ring + W_STAGES * W_BYTES);
             for (int tile = first; tile < tiles; tile += stride) {
                 for (int sl = 0; sl < n_sl; ++sl) {
@@ -363,7 +363,7 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         if ((st * SR) % GS == 0 && !mbar_wait_warp(smem_u32(&sh.d_empty[db]), dph, abort_flag)) return;
                         if (!mbar_wait_warp(smem_u32(&sh.a_full[ab]), aph, abort_flag)) return;
                         tc_fence_after();
-                        const uint32_t a = tmem_base + ab * (SR * 16), d = tmem_base + d_col_of(NT) + db * (SR * NT);
+                        const uint32_t a = tmem_base + ab * (SR * 16), d = tmem_base + rq_w4_d_col(NT) + db * (SR * NT);
 #pragma unroll
                         for (int i = 0; i < SR; ++i) {
                             const int r = st * SR + i;
@@ -375,7 +375,8 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         umma_commit(smem_u32(&sh.a_empty[ab]));
                         if (++ab == NA) { ab = 0; aph ^= 1u; }
                         if ((st * SR + SR) % GS == 0) {
-                            umma_commit(smem_u32(&sh.d_full[db]));
+                            umma_commit(smem_u32(&sh.d_full[NF == ND ? db : fb]));
+                            if (NF != ND && ++fb == NF) fb = 0;
                             if (++db == ND) { db = 0; dph ^= 1u; }
                         }
                     }
@@ -436,7 +437,7 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // ---- fold
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const int q = warp & 3, h = (warp - 4 - UNPACK_WARPS) >> 2, row = q * 32 + lane;
-        const uint32_t lane_base = tmem_base + ((uint32_t) (q * 32) << 16) + d_col_of(NT);
+        const uint32_t lane_base = tmem_base + ((uint32_t) (q * 32) << 16) + rq_w4_d_col(NT);
         const bool fmt_ok = prm.status == nullptr || prm.status[1] == RQ_FMT_I8;
         if (!fmt_ok && threadIdx.x == (4 + UNPACK_WARPS) * 32) atomicExch(prm.status, 2);
         uint32_t gset = 0, it = 0;            // accumulator sets and slices, all tiles
@@ -460,7 +461,7 @@ rq_gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     if (HAS_K) k4 = __ldg(reinterpret_cast<const uint32_t *>(kp) + sl);      // four multipliers, one per run
                     if (!mbar_wait_warp(smem_u32(&sh.m_full[ms]), (it / MS) & 1u, abort_flag)) { ok = false; break; }
                     const uint32_t db = gset % ND;
-                    if (!mbar_wait_warp(smem_u32(&sh.d_full[db]), (gset / ND) & 1u, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(smem_u32(&sh.d_full[gset % NF]), (gset / NF) & 1u, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     for (int g = 0; g < dgroups; g += CG) {
                         int v[CG][NT];
