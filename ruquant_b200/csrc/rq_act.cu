@@ -88,11 +88,18 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P) : 1)
     if (t == 0 && tid == 0 && prm.status != nullptr) prm.status[1] = prm.fmt;     // word 0 (errors) is sticky: only the host clears it
     RQ_STAMP(tid == 0);                                     // 1: after the wait
 
-    // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
     const float * xrow = prm.x + (int64_t) t * prm.ldx;
-    if (!bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid)) {
-        if (tid == 0 && prm.status != nullptr) atomicExch(prm.status, 1);
-        return;
+    if (prm.status != nullptr) {
+        // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
+        if (!bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid)) {
+            if (tid == 0) atomicExch(prm.status, 1);
+            return;
+        }
+    } else {
+        // a rotation without a workspace has nowhere to report a wait that ran out: plain loads, nothing to wait for
+#pragma unroll 4
+        for (int i = tid; i < K / 4; i += nt) reinterpret_cast<float4 *>(buf)[i] = __ldg(reinterpret_cast<const float4 *>(xrow) + i);
+        __syncthreads();
     }
     if (prm.n_rot > 0) {
         fwht_resident(buf, K, prm.m, tid, nt);

@@ -18,7 +18,6 @@
 #include <math.h>
 
 #include "rq_common.cuh"
-#include "rq_act_dev.cuh"
 
 namespace {
 
@@ -125,20 +124,16 @@ __global__ void __launch_bounds__(WROW_THREADS) rq_wrow_kernel(const float * __r
     __shared__ int red_i[WROW_THREADS / 32];
     __shared__ float win_s;
     __shared__ unsigned contested_s;
-    __shared__ uint64_t row_bar;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t row = blockIdx.x;
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((uint32_t) __cvta_generic_to_shared(&row_bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
     const float * xr = x + row * ldx;
-    if (!rq_act_dev::bulk_load_row(xs, xr, (uint32_t) K * 4u, &row_bar, tid)) return;      // (the bounded wait ran out: no block is written)
 
+    // (plain loads: a bulk copy would have to be awaited, and a conversion has nowhere to report a wait that ran out)
     float amax = 0.0f;
+#pragma unroll 4
     for (int i = tid; i < K / 4; i += WROW_THREADS) {
-        const float4 q = reinterpret_cast<const float4 *>(xs)[i];
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(xr) + i);
+        reinterpret_cast<float4 *>(xs)[i] = q;
         amax = fmaxf(fmaxf(fmaxf(amax, fabsf(q.x)), fmaxf(fabsf(q.y), fabsf(q.z))), fabsf(q.w));
     }
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
