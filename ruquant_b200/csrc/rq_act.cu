@@ -91,10 +91,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P) : 1)
     const float * xrow = prm.x + (int64_t) t * prm.ldx;
     if (prm.status != nullptr) {
         // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
-        if (!bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid)) {
-            if (tid == 0) atomicExch(prm.status, 1);
-            return;
-        }
+        bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid, prm.status);
     } else {
         // a rotation without a workspace has nowhere to report a wait that ran out: plain loads, nothing to wait for
 #pragma unroll 4

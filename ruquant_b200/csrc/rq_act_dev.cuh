@@ -314,24 +314,37 @@ __device__ __forceinline__ void fwht_resident(float * buf, int len, int m, int t
     }
 }
 
+// Whether the copy that completes phase 0 of `bar` has landed; false when it has not within `cycles`.
+__device__ __forceinline__ bool row_landed(uint32_t bar, long long cycles) {
+    const long long t0 = clock64();
+    for (uint32_t i = 0;; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar) : "memory");
+        if (ok) return true;
+        if ((i & 63u) == 63u && clock64() - t0 > cycles) return false;
+    }
+}
+// The wait for it, by every thread of the CTA.  A thread whose wait runs out (about a second) sets the error word and waits once
+// more, so that the CTA does not end under a copy that is still in flight; then it goes on with what the buffer holds.  No thread
+// leaves: others may have seen the copy land, and the barriers and shuffles that follow are for all of them.  (Whatever the
+// floats, codes are bytes and every index is in range; the error word says that the results are not to be used.)
+__device__ __forceinline__ void await_row(uint32_t bar, int32_t * status, long long cycles = 2000000000ll) {
+    if (row_landed(bar, cycles)) return;
+    atomicExch(status, 1);
+    row_landed(bar, cycles);
+}
 // One bulk asynchronous copy of a row (bytes a multiple of 16, both ends 16-byte aligned) into shared memory, issued by
 // one thread, awaited by all: a single trip to memory for the whole row, where per-run loads expose one trip per round of
-// runs a warp takes.  The wait is bounded (about a second); false when it ran out.
-__device__ __forceinline__ bool bulk_load_row(float * dst, const float * src, uint32_t bytes, uint64_t * bar, int tid) {
+// runs a warp takes.
+__device__ __forceinline__ void bulk_load_row(float * dst, const float * src, uint32_t bytes, uint64_t * bar, int tid, int32_t * status) {
     const uint32_t b = (uint32_t) __cvta_generic_to_shared(bar);
     if (tid == 0) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(bytes) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"(bytes), "r"(b) : "memory");
     }
-    const long long t0 = clock64();
-    for (uint32_t i = 0;; ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(b) : "memory");
-        if (ok) return true;
-        if ((i & 63u) == 63u && clock64() - t0 > 2000000000ll) return false;
-    }
+    await_row(b, status);
 }
 
 // A buffer of `len` floats made of whole chunks of m: loaded from global memory and Sylvester-transformed chunk by
