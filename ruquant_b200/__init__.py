@@ -125,6 +125,16 @@ def _stream_ptr(stream=None):
     return ctypes.c_void_p(stream.cuda_stream)
 
 
+def _empty_on(stream, nbytes, device):
+    """Bytes for one call's own use on `stream` (None: the current one).  They come from that stream's pool: memory of another
+    stream's would be handed on, when the call returns and drops it, while the call's kernels still run."""
+    import torch
+    if stream is None:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    with torch.cuda.stream(stream):
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 # array types of a call's weights: pointers to descriptors, output addresses, row strides
 _DESCS, _PTRS, _I64S = [[t * n for n in range(4)] for t in (ctypes.POINTER(WeightDesc), ctypes.c_void_p, ctypes.c_int64)]
 
@@ -210,6 +220,9 @@ def mul_mat(weights, x, out=None, clip=None, act_group=None, path=PATH_AUTO, wor
     device = x.device
     if out is None:
         outs = [torch.empty((M, w.N), dtype=torch.float32, device=device) for w in ws_list]
+        if stream is not None:
+            for o in outs:
+                o.record_stream(stream)
     else:
         outs = [out] if single else list(out)
     if clip is None:
@@ -230,12 +243,9 @@ def mul_mat(weights, x, out=None, clip=None, act_group=None, path=PATH_AUTO, wor
     def call():
         ws = workspace
         if ws is None:
-            if stream is None:
-                # used by this call alone, on the stream that its status block is zeroed on: nothing to wait for
-                ws = torch.empty(workspace_bytes(K, M), dtype=torch.uint8, device=device)
-                _check(L.rq_w4a4_workspace_init(ws.data_ptr(), K, M, handle), "rq_w4a4_workspace_init")
-            else:
-                ws = new_workspace(K, M, device)
+            # used by this call alone, on the stream that its status block is zeroed on: nothing to wait for
+            ws = _empty_on(stream, workspace_bytes(K, M), device)
+            _check(L.rq_w4a4_workspace_init(ws.data_ptr(), K, M, handle), "rq_w4a4_workspace_init")
         _check(L.rq_w4a4_mul_mat(descs, n_w, x.data_ptr(), x.stride(0), M, ys, ldy, clip, act_group, path, ws.data_ptr(), ws.numel(),
                                  handle), "rq_w4a4_mul_mat")
 
@@ -372,8 +382,10 @@ def quantize_weights(w, type_, wgroup=0, rot_blocks=1, stream=None):
     if nbytes == 0:
         raise RqError(-2, "rq_w4a4_quantize_weights_scratch_bytes")
     with torch.cuda.device(w.device):
-        scratch = torch.empty(nbytes, dtype=torch.uint8, device=w.device)
+        scratch = _empty_on(stream, nbytes, w.device)
         out = torch.empty((N, K // BLOCK_CODES * BLOCK_BYTES), dtype=torch.uint8, device=w.device)
+        if stream is not None:
+            out.record_stream(stream)
         _check(lib().rq_w4a4_quantize_weights(w.data_ptr(), w.stride(0), type_, K, N, wgroup, rot_blocks, out.data_ptr(),
                                               scratch.data_ptr(), nbytes, _stream_ptr(stream)), "rq_w4a4_quantize_weights")
     return out
