@@ -31,6 +31,7 @@
 
 #include "rq_common.cuh"
 #include "rq_act_dev.cuh"
+#include "rq_act_plan.h"
 
 namespace cg = cooperative_groups;
 
@@ -379,7 +380,7 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
     static std::mutex mu;
     static bool configured[64] = {};
     static int sms[64] = {};
-    static int at_once[64][17] = {};       // clusters of 2, 4 and 8 CTAs that run at once
+    static int at_once[64][9] = {};       // clusters of 2, 4 and 8 CTAs that run at once
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -402,9 +403,8 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
         const int units = (K / prm.n_rot) * (prm.m / 64) * (CP / 4);
         // the widest cluster of which all M run at once: a second round costs more than the narrower cluster (16 tokens of 17408:
         // 17.1 us with 8 CTAs a token, 10.3 with 4; 5120: 8.0 and 4.4; 64 tokens of 17408 with 2: 15.6, one CTA a token: 16.7)
-        static const int c_max = rq_env_int("RQ_TUNE_ACT_CMAX", 8);
-        int C = c_max;
-        while (C > 1 && (units < 2 * C || M > at_once[dev][C])) C >>= 1;
+        static const int cap = rq_act_cluster_cap(rq_env_int("RQ_TUNE_ACT_CMAX", 8));
+        const int C = rq_act_cluster(cap, units, M, at_once[dev]);
         const int units_max = (units + C - 1) / C;
         const size_t smem = ((size_t) K + (size_t) CP * CP + (size_t) units_max * 4 * 64) * sizeof(float);
         if (C > 1 && smem <= SMEM_LIMIT) {
