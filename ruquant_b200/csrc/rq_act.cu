@@ -94,9 +94,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P) : 1)
         // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
         bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid, prm.status);
     } else {
-        // a rotation without a workspace has nowhere to report a wait that ran out: plain loads, nothing to wait for
-#pragma unroll 4
-        for (int i = tid; i < K / 4; i += nt) reinterpret_cast<float4 *>(buf)[i] = __ldg(reinterpret_cast<const float4 *>(xrow) + i);
+        copy_row(buf, xrow, K, tid, nt);           // (a rotation without a workspace has nowhere to report a wait that ran out)
         __syncthreads();
     }
     if (prm.n_rot > 0) {

@@ -347,6 +347,16 @@ __device__ __forceinline__ void bulk_load_row(float * dst, const float * src, ui
     await_row(b, status);
 }
 
+// A row by 16-byte asynchronous copies of every thread, all of them in flight at once and waited for as loads are: no barrier
+// word, nothing that could run out.  A thread sees the pieces tid, tid + nt, ... that it copied itself, the others behind a
+// CTA barrier.
+__device__ __forceinline__ void copy_row(float * dst, const float * src, int len, int tid, int nt) {
+    const uint32_t d = (uint32_t) __cvta_generic_to_shared(dst);
+    for (int i = tid; i < len / 4; i += nt)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(d + (uint32_t) i * 16u), "l"(src + 4 * i) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // A buffer of `len` floats made of whole chunks of m: loaded from global memory and Sylvester-transformed chunk by
 // chunk.  Chunks up to 1024 wide are done entirely in registers and shuffles; wider chunks finish their upper
 // strides (1024 and above, conflict-free) in shared memory.  Ends with a CTA barrier.

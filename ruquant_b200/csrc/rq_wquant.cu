@@ -18,6 +18,7 @@
 #include <math.h>
 
 #include "rq_common.cuh"
+#include "rq_act_dev.cuh"
 
 namespace {
 
@@ -128,12 +129,12 @@ __global__ void __launch_bounds__(WROW_THREADS) rq_wrow_kernel(const float * __r
     const int64_t row = blockIdx.x;
     const float * xr = x + row * ldx;
 
-    // (plain loads: a bulk copy would have to be awaited, and a conversion has nowhere to report a wait that ran out)
-    float amax = 0.0f;
-#pragma unroll 4
+    // (not by a bulk copy, whose wait may run out: a conversion has nowhere to report that)
+    rq_act_dev::copy_row(xs, xr, K, tid, WROW_THREADS);
+
+    float amax = 0.0f;                            // (of the pieces this thread copied: no barrier yet)
     for (int i = tid; i < K / 4; i += WROW_THREADS) {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(xr) + i);
-        reinterpret_cast<float4 *>(xs)[i] = q;
+        const float4 q = reinterpret_cast<const float4 *>(xs)[i];
         amax = fmaxf(fmaxf(fmaxf(amax, fabsf(q.x)), fmaxf(fabsf(q.y), fabsf(q.z))), fabsf(q.w));
     }
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
