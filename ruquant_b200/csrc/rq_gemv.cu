@@ -61,6 +61,7 @@ __device__ __forceinline__ int job_of_tile(const GemvParams & prm, int tile) {
 }
 
 constexpr int CH_STEPS = 4;                 // 64-input steps per chunk of the stream
+static_assert(CH_STEPS == 4, "a chunk's weight multipliers of a row are one aligned 32-bit word");
 constexpr int CH_BYTES = CH_STEPS * 512;    // 2 KB: the unit one consumer warp works on
 constexpr int SUBS = 4;                     // chunks per bulk copy
 constexpr int ST_BYTES = SUBS * CH_BYTES;   // 8 KB per bulk copy: few enough copies for a single issuing thread
@@ -200,9 +201,14 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
             const int c = st * SUBS + sc;                 // this warp's chunk of the tile (may lie beyond its end)
             // the activations do not depend on the weights: fetch them while the stage is still in flight
             uint4 bq[CH_STEPS];
+            uint32_t k4_lo = 0, k4_hi = 0;                // the chunk's four weight multipliers of a row in one word
             if (c < nchunks) {
 #pragma unroll
                 for (int q = 0; q < CH_STEPS; ++q) bq[q] = __ldg(ap + (c * CH_STEPS + q) * 4);
+                if (HAS_K) {
+                    k4_lo = __ldg(reinterpret_cast<const uint32_t *>(kp_lo) + c);
+                    k4_hi = __ldg(reinterpret_cast<const uint32_t *>(kp_hi) + c);
+                }
             }
             // the MMAs below are warp-collective: leave the loop together or not at all
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (gs / STAGES) & 1, abort_flag))) { ok = false; break; }
@@ -232,8 +238,9 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
                 }
                 if ((st % GS) == GS - 1) {
                     const int ag = j / GS;
-                    int klo = 1, khi = 1;
-                    if (HAS_K) { klo = kp_lo[j]; khi = kp_hi[j]; }
+                    // (asked for with the activations: a byte load each here, behind the MMAs, takes 44 us instead of 27 for 8 tokens
+                    // of 17408 x 8192)
+                    const int klo = (int) ((k4_lo >> (8 * st)) & 0xFFu), khi = (int) ((k4_hi >> (8 * st)) & 0xFFu);
                     const int m0 = __ldg(mp[0] + ag);
                     const int m1 = ONE ? 0 : __ldg(mp[1] + ag);
                     if (HAS_K) {
@@ -310,7 +317,11 @@ cudaError_t launch_one(const GemvParams & prm, cudaStream_t stream) {
     static std::mutex mu;
     static bool configured[64] = {};
     static int per_sm[64] = {};
-    const size_t smem = (size_t) STAGES * ST_BYTES + 2 * (size_t) CONSUMERS * 32 * 4 * sizeof(int);
+    // With multipliers and several tokens the folds are a third longer and three CTAs an SM are no faster than two, which share
+    // out the tiles more evenly: the padding admits two (8 tokens of 6144 x 8192: 11.6 us with three, 8.9 with two; 17408 x
+    // 8192: 27 and 20).
+    constexpr size_t pad = HAS_K && GS == 1 && !ONE && !PUSH ? 14 * 1024 : 0;
+    const size_t smem = pad + (size_t) STAGES * ST_BYTES + 2 * (size_t) CONSUMERS * 32 * 4 * sizeof(int);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
