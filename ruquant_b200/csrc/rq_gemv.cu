@@ -1,9 +1,10 @@
-// Decode-width contraction (up to 8 tokens; rq_gemm_w4.cu takes 9 to 64): an HBM-bound GEMV over the int4 decode stream.
+// Decode-width contraction (up to 8 tokens, up to 16 where rq_gemv_plan.h says so; rq_gemm_w4.cu takes the rest up to 64): an
+// HBM-bound GEMV over the int4 decode stream.
 //
 // The stream is stored in the order the warp consumes it (rq_prepack.cu): for every tile of 16 weight rows and every
 // run of 64 inputs, 512 contiguous bytes = one 128-bit load per lane, whose four words unpack (two logic ops each)
 // into the eight int8 A-fragment registers of two m16n8k32 integer MMAs.  The MMAs do the multiply-accumulate for
-// up to 8 tokens at once, so only the folds grow with M.  Every activation group of every (row, token) pair is folded on its own, as
+// up to 8 tokens at once (two of them 16), so only the folds grow with M.  Every activation group of every (row, token) pair is folded on its own, as
 // the reference's dot product does (ggml_vec_dot_w4a4_a4, ggml/src/ggml-cpu/quants.c in
 // patches/llama.cpp-ruquant.patch:148-177):
 //     total += (k * m_g * S_g) >> 4,   S_g = sum c * (q - z_g)       (int32, arithmetic shift)
@@ -19,6 +20,7 @@
 #include <mutex>
 
 #include "rq_common.cuh"
+#include "rq_gemv_plan.h"
 
 namespace {
 
@@ -93,16 +95,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // warp streams the tiles' K/64 * 512 bytes back to back into a shared-memory ring with bulk copies (it starts at once:
 // the weights do not depend on the preceding kernel, and it never drains between tiles); the consumer warps take the
 // chunks of that stream round-robin, so 64 KB per CTA stay in flight or resident from the first cycle to the last.
-// GS: 64-input steps per activation group (1, 2, 4).  HAS_K: weight multipliers.
+// NT: token tiles of 8 (1 or 2).  GS: 64-input steps per activation group (1, 2, 4).  HAS_K: weight multipliers.
 // ONE: M == 1 (only token 0 is folded and stored).  PUSH: outputs also go to the jobs' further destinations.
-template <int GS, bool HAS_K, bool ONE, bool PUSH>
+template <int NT, int GS, bool HAS_K, bool ONE, bool PUSH>
 __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const GemvParams prm) {
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ uint64_t full[STAGES], empty[STAGES];
     __shared__ int abort_word;
     __shared__ int fmt_word;     // the activation format the quantizer recorded (-1 until a spare producer lane has read it)
     uint8_t * ring = dyn;
-    int * part = reinterpret_cast<int *>(dyn + STAGES * ST_BYTES);      // [2][CONSUMERS][32][4]
+    int * part = reinterpret_cast<int *>(dyn + STAGES * ST_BYTES);      // [2][CONSUMERS][32][4 * NT]
     volatile int * abort_flag = &abort_word;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gid = lane >> 2, tig = lane & 3;
@@ -172,13 +174,20 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) rq_trace(prm.status, 0x11);
 
-    // B fragments: token gid; the quantizer stores each run of 64 inputs so that the 16
+    // B fragments: token gid (+8 for the second tile); the quantizer stores each run of 64 inputs so that the 16
     // bytes at offset tig*16 are inputs {0,16,32,48} + tig*4 .. +3: b0, b1 of both MMAs in one 128-bit load.
     // Token slots beyond M read token 0's data: their columns of the product are never stored.
-    const uint4 * ap = reinterpret_cast<const uint4 *>(prm.a8 + (size_t) (gid < M ? gid : 0) * K) + tig;
-    const int32_t * mp[2];
+    const uint4 * ap[NT];
+    const int32_t * mp[NT][2];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) mp[c] = prm.msh + (size_t) (2 * tig + c < M ? 2 * tig + c : 0) * n_ag;
+    for (int t = 0; t < NT; ++t) {
+        ap[t] = reinterpret_cast<const uint4 *>(prm.a8 + (size_t) (gid + 8 * t < M ? gid + 8 * t : 0) * K) + tig;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int tok = 8 * t + 2 * tig + c;
+            mp[t][c] = prm.msh + (size_t) (tok < M ? tok : 0) * n_ag;
+        }
+    }
 
     int it = 0;                                    // tiles done by this CTA
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
@@ -190,7 +199,11 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
             kp_lo = jb.wk + (size_t) (row_lo < jb.N ? row_lo : 0) * ng64;
             kp_hi = jb.wk + (size_t) (row_hi < jb.N ? row_hi : 0) * ng64;
         }
-        int tot[4] = { 0, 0, 0, 0 }, acc[4] = { 0, 0, 0, 0 };
+        int tot[NT][4], acc[NT][4];
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) tot[t][i] = acc[t][i] = 0;
 
         // stage gs of the CTA's stream (all tiles) is shared by four consumer warps, one chunk each: warps 0-3 take
         // the even stages, warps 4-7 the odd ones
@@ -200,11 +213,13 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
             const int gs = gs0 + st, s = gs % STAGES;
             const int c = st * SUBS + sc;                 // this warp's chunk of the tile (may lie beyond its end)
             // the activations do not depend on the weights: fetch them while the stage is still in flight
-            uint4 bq[CH_STEPS];
+            uint4 bq[CH_STEPS][NT];
             uint32_t k4_lo = 0, k4_hi = 0;                // the chunk's four weight multipliers of a row in one word
             if (c < nchunks) {
 #pragma unroll
-                for (int q = 0; q < CH_STEPS; ++q) bq[q] = __ldg(ap + (c * CH_STEPS + q) * 4);
+                for (int q = 0; q < CH_STEPS; ++q)
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) bq[q][t] = __ldg(ap[t] + (c * CH_STEPS + q) * 4);
                 if (HAS_K) {
                     k4_lo = __ldg(reinterpret_cast<const uint32_t *>(kp_lo) + c);
                     k4_hi = __ldg(reinterpret_cast<const uint32_t *>(kp_hi) + c);
@@ -214,53 +229,62 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (gs / STAGES) & 1, abort_flag))) { ok = false; break; }
             if (c < nchunks) {
             const uint4 * sp_ = reinterpret_cast<const uint4 *>(ring + (size_t) s * ST_BYTES + (size_t) sc * CH_BYTES) + rq_w4_slot(gid, tig);
-            // The integer MMA of this part has a long latency: issue the MMAs of all steps of the chunk (two per step, on
+            // The integer MMA of this part has a long latency: issue the MMAs of SP steps (two per step and token tile, on
             // independent zero-initialised accumulators) before touching any result.
-            int pa[CH_STEPS][2][4];
+            constexpr int SP = NT == 1 ? CH_STEPS : CH_STEPS / 2;
 #pragma unroll
-            for (int sp = 0; sp < CH_STEPS; ++sp) {
-                const uint4 wv = sp_[sp * 32], b = bq[sp];
-                // words 0, 1: row gid, first and second 32 inputs; words 2, 3: row gid + 8
-                const int a0[4] = { (int) ((wv.x << 4) & 0xF0F0F0F0u), (int) ((wv.z << 4) & 0xF0F0F0F0u), (int) (wv.x & 0xF0F0F0F0u), (int) (wv.z & 0xF0F0F0F0u) };
-                const int a1[4] = { (int) ((wv.y << 4) & 0xF0F0F0F0u), (int) ((wv.w << 4) & 0xF0F0F0F0u), (int) (wv.y & 0xF0F0F0F0u), (int) (wv.w & 0xF0F0F0F0u) };
-                const int zero[4] = { 0, 0, 0, 0 };
-                mma_s8(pa[sp][0], a0, (int) b.x, (int) b.y, zero);
-                mma_s8(pa[sp][1], a1, (int) b.z, (int) b.w, zero);
-            }
+            for (int h = 0; h < CH_STEPS; h += SP) {
+                int pa[SP][2][NT][4];
 #pragma unroll
-            for (int st = 0; st < CH_STEPS; ++st) {
-                const int j = c * CH_STEPS + st;
+                for (int sp = 0; sp < SP; ++sp) {
+                    const uint4 wv = sp_[(h + sp) * 32];
+                    // words 0, 1: row gid, first and second 32 inputs; words 2, 3: row gid + 8
+                    const int a0[4] = { (int) ((wv.x << 4) & 0xF0F0F0F0u), (int) ((wv.z << 4) & 0xF0F0F0F0u), (int) (wv.x & 0xF0F0F0F0u), (int) (wv.z & 0xF0F0F0F0u) };
+                    const int a1[4] = { (int) ((wv.y << 4) & 0xF0F0F0F0u), (int) ((wv.w << 4) & 0xF0F0F0F0u), (int) (wv.y & 0xF0F0F0F0u), (int) (wv.w & 0xF0F0F0F0u) };
+                    const int zero[4] = { 0, 0, 0, 0 };
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (ONE && (i & 1)) continue;                 // token 1 of the pair does not exist
-                    if (GS == 1) acc[i] = pa[st][0][i] + pa[st][1][i];
-                    else         acc[i] += pa[st][0][i] + pa[st][1][i];
-                }
-                if ((st % GS) == GS - 1) {
-                    const int ag = j / GS;
-                    // (asked for with the activations: a byte load each here, behind the MMAs, takes 44 us instead of 27 for 8 tokens
-                    // of 17408 x 8192)
-                    const int klo = (int) ((k4_lo >> (8 * st)) & 0xFFu), khi = (int) ((k4_hi >> (8 * st)) & 0xFFu);
-                    const int m0 = __ldg(mp[0] + ag);
-                    const int m1 = ONE ? 0 : __ldg(mp[1] + ag);
-                    if (HAS_K) {
-                        tot[0] += (klo * m0 * (acc[0] >> 7)) >> 4;
-                        tot[2] += (khi * m0 * (acc[2] >> 7)) >> 4;
-                        if (!ONE) {
-                            tot[1] += (klo * m1 * (acc[1] >> 7)) >> 4;
-                            tot[3] += (khi * m1 * (acc[3] >> 7)) >> 4;
-                        }
-                    } else {
-                        tot[0] += (m0 * acc[0]) >> RQ_FOLD_SHIFT;
-                        tot[2] += (m0 * acc[2]) >> RQ_FOLD_SHIFT;
-                        if (!ONE) {
-                            tot[1] += (m1 * acc[1]) >> RQ_FOLD_SHIFT;
-                            tot[3] += (m1 * acc[3]) >> RQ_FOLD_SHIFT;
-                        }
+                    for (int t = 0; t < NT; ++t) {
+                        const uint4 b = bq[h + sp][t];
+                        mma_s8(pa[sp][0][t], a0, (int) b.x, (int) b.y, zero);
+                        mma_s8(pa[sp][1][t], a1, (int) b.z, (int) b.w, zero);
                     }
-                    if (GS > 1) {
+                }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) acc[i] = 0;
+                for (int sp = 0; sp < SP; ++sp) {
+                    const int st = h + sp, ag = (c * CH_STEPS + st) / GS;
+                    // (asked for with the activations: a byte load each here, behind the MMAs, takes 44 us instead of 27 for 8 tokens of
+                    // 17408 x 8192)
+                    const int klo = (int) ((k4_lo >> (8 * st)) & 0xFFu), khi = (int) ((k4_hi >> (8 * st)) & 0xFFu);
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (ONE && (i & 1)) continue;                 // token 1 of the pair does not exist
+                            if (GS == 1) acc[t][i] = pa[sp][0][t][i] + pa[sp][1][t][i];
+                            else         acc[t][i] += pa[sp][0][t][i] + pa[sp][1][t][i];
+                        }
+                        if ((st % GS) != GS - 1) continue;
+                        const int m0 = __ldg(mp[t][0] + ag);
+                        const int m1 = ONE ? 0 : __ldg(mp[t][1] + ag);
+                        if (HAS_K) {
+                            tot[t][0] += (klo * m0 * (acc[t][0] >> 7)) >> 4;
+                            tot[t][2] += (khi * m0 * (acc[t][2] >> 7)) >> 4;
+                            if (!ONE) {
+                                tot[t][1] += (klo * m1 * (acc[t][1] >> 7)) >> 4;
+                                tot[t][3] += (khi * m1 * (acc[t][3] >> 7)) >> 4;
+                            }
+                        } else {
+                            tot[t][0] += (m0 * acc[t][0]) >> RQ_FOLD_SHIFT;
+                            tot[t][2] += (m0 * acc[t][2]) >> RQ_FOLD_SHIFT;
+                            if (!ONE) {
+                                tot[t][1] += (m1 * acc[t][1]) >> RQ_FOLD_SHIFT;
+                                tot[t][3] += (m1 * acc[t][3]) >> RQ_FOLD_SHIFT;
+                            }
+                        }
+                        if (GS > 1) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) acc[t][i] = 0;
+                        }
                     }
                 }
             }
@@ -271,18 +295,22 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
 
         // combine the consumer warps (integer sums are exact in any order); partials are double-buffered by tile
         // parity, and the warp that reduces and stores rotates from tile to tile
-        int * pt = part + (it & 1) * (CONSUMERS * 32 * 4);
+        int * pt = part + (it & 1) * (CONSUMERS * 32 * 4 * NT);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pt[(warp * 32 + lane) * 4 + i] = tot[i];
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pt[(warp * 32 + lane) * 4 * NT + t * 4 + i] = tot[t][i];
         asm volatile("bar.sync 1, %0;" :: "n"(CONSUMERS * 32) : "memory");
         if (!ok || *abort_flag) return;
         if (warp != it % CONSUMERS) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int v = 0;
-            for (int w = 0; w < CONSUMERS; ++w) v += pt[(w * 32 + lane) * 4 + i];
-            tot[i] = v;
-        }
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                int v = 0;
+                for (int w = 0; w < CONSUMERS; ++w) v += pt[(w * 32 + lane) * 4 * NT + t * 4 + i];
+                tot[t][i] = v;
+            }
         int fmt = *reinterpret_cast<volatile int *>(&fmt_word);
         for (int spin = 0; fmt < 0 && spin < (1 << 20); ++spin) fmt = *reinterpret_cast<volatile int *>(&fmt_word);
         const bool fmt_ok = fmt == RQ_FMT_I8;
@@ -290,12 +318,12 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
         const float s_lo = row_lo < jb.N ? __ldg(jb.sw + row_lo) : 0.0f;
         const float s_hi = row_hi < jb.N ? __ldg(jb.sw + row_hi) : 0.0f;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int tok = 2 * tig + c;
+        for (int tc = 0; tc < 2 * NT; ++tc) {
+            const int t = tc >> 1, c = tc & 1, tok = 8 * t + 2 * tig + c;
             if (tok < M && fmt_ok) {
                 const float ut = __ldg(prm.u + tok);
-                const float v_lo = __fmul_rn(__fmul_rn(__fmul_rn((float) tot[c], 16.0f), ut), s_lo);
-                const float v_hi = __fmul_rn(__fmul_rn(__fmul_rn((float) tot[2 + c], 16.0f), ut), s_hi);
+                const float v_lo = __fmul_rn(__fmul_rn(__fmul_rn((float) tot[t][c], 16.0f), ut), s_lo);
+                const float v_hi = __fmul_rn(__fmul_rn(__fmul_rn((float) tot[t][2 + c], 16.0f), ut), s_hi);
                 if (row_lo < jb.N) jb.y[(size_t) tok * jb.ldy + row_lo] = v_lo;
                 if (row_hi < jb.N) jb.y[(size_t) tok * jb.ldy + row_hi] = v_hi;
                 // N-sharded ranks: the same values straight into every other rank's copy of the output
@@ -311,47 +339,60 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const
     if (threadIdx.x == 0) rq_trace(prm.status, 0x13);
 }
 
-template <int GS, bool HAS_K, bool ONE, bool PUSH>
-cudaError_t launch_one(const GemvParams & prm, cudaStream_t stream) {
-    // first use of this instantiation on a device; several host threads may get here at once
-    static std::mutex mu;
-    static bool configured[64] = {};
-    static int per_sm[64] = {};
+template <int NT, int GS, bool HAS_K, bool ONE, bool PUSH>
+constexpr size_t gemv_smem() {
     // With multipliers and several tokens the folds are a third longer and three CTAs an SM are no faster than two, which share
     // out the tiles more evenly: the padding admits two (8 tokens of 6144 x 8192: 11.6 us with three, 8.9 with two; 17408 x
     // 8192: 27 and 20).
-    constexpr size_t pad = HAS_K && GS == 1 && !ONE && !PUSH ? 14 * 1024 : 0;
-    const size_t smem = pad + (size_t) STAGES * ST_BYTES + 2 * (size_t) CONSUMERS * 32 * 4 * sizeof(int);
+    constexpr size_t pad = NT == 1 && HAS_K && GS == 1 && !ONE && !PUSH ? 14 * 1024 : 0;
+    return pad + (size_t) STAGES * ST_BYTES + 2 * (size_t) CONSUMERS * 32 * 4 * NT * sizeof(int);
+}
+
+// CTAs of an instantiation that run at once, less those whose place the kernel ahead may still hold
+template <int NT, int GS, bool HAS_K, bool ONE, bool PUSH>
+cudaError_t resident_ctas(int * n) {
+    // first use of this instantiation on a device; several host threads may get here at once
+    static std::mutex mu;
+    static bool configured[64] = {};
+    static int per_device[64] = {};
+    constexpr size_t smem = gemv_smem<NT, GS, HAS_K, ONE, PUSH>();
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    int resident_slots;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!configured[dev]) {
-            e = cudaFuncSetAttribute(rq_gemv_mma_kernel<GS, HAS_K, ONE, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-            if (e != cudaSuccess) return e;
-            // persistent grid: as many CTAs as are resident at once
-            int nb = 0, sms = 148;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rq_gemv_mma_kernel<GS, HAS_K, ONE, PUSH>, (CONSUMERS + 1) * 32, smem);
-            if (e != cudaSuccess) return e;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            per_sm[dev] = (nb > 0 ? nb : 1) * sms;
-            configured[dev] = true;
-        }
-        resident_slots = per_sm[dev];
-    }
-    cudaLaunchConfig_t cfg = {};
-    const int tiles = prm.tile_start[prm.n_jobs];
     // The quantizer ahead of this kernel (a cluster of up to 8 CTAs per token) still holds its shared memory when this
     // grid starts: CTAs beyond the free slots would start only after it, with their whole share of tiles still to do.
     static const int reserve = rq_env_int("RQ_TUNE_GEMV_RESERVE", 8);
-    const int resident = resident_slots - reserve;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!configured[dev]) {
+        e = cudaFuncSetAttribute(rq_gemv_mma_kernel<NT, GS, HAS_K, ONE, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        if (e != cudaSuccess) return e;
+        // persistent grid: as many CTAs as are resident at once
+        int nb = 0, sms = 148;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rq_gemv_mma_kernel<NT, GS, HAS_K, ONE, PUSH>, (CONSUMERS + 1) * 32, smem);
+        if (e != cudaSuccess) return e;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        per_device[dev] = (nb > 0 ? nb : 1) * sms;
+        configured[dev] = true;
+    }
+    *n = per_device[dev] - reserve;
+    return cudaSuccess;
+}
+
+// taken: false when the tensor-core kernel is the better one for this launch (nothing is launched then)
+template <int NT, int GS, bool HAS_K, bool ONE, bool PUSH>
+cudaError_t launch_one(const GemvParams & prm, cudaStream_t stream, bool * taken) {
+    int resident = 0;
+    const cudaError_t e = resident_ctas<NT, GS, HAS_K, ONE, PUSH>(&resident);
+    if (e != cudaSuccess) return e;
+    const int tiles = prm.tile_start[prm.n_jobs];
+    *taken = NT == 1 || rq_gemv_takes_16(prm.K, tiles, resident, prm.M);
+    if (!*taken) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
     // (an evenly divided grid -- every CTA the same number of tiles -- measured slower: 3.79 against 3.68 ms per pass)
     cfg.gridDim = dim3((unsigned) (tiles < resident ? tiles : resident));
     cfg.blockDim = dim3((CONSUMERS + 1) * 32);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = gemv_smem<NT, GS, HAS_K, ONE, PUSH>();
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -359,27 +400,28 @@ cudaError_t launch_one(const GemvParams & prm, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = pdl;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, rq_gemv_mma_kernel<GS, HAS_K, ONE, PUSH>, prm);
+    return cudaLaunchKernelEx(&cfg, rq_gemv_mma_kernel<NT, GS, HAS_K, ONE, PUSH>, prm);
 }
 
-template <int GS, bool HAS_K>
-cudaError_t launch(const GemvParams & prm, cudaStream_t stream) {
+template <int NT, int GS, bool HAS_K>
+cudaError_t launch(const GemvParams & prm, cudaStream_t stream, bool * taken) {
     bool push = false;
     for (int i = 0; i < prm.n_jobs; ++i) push = push || prm.job[i].n_more > 0;
-    if (prm.M == 1) return push ? launch_one<GS, HAS_K, true, true>(prm, stream) : launch_one<GS, HAS_K, true, false>(prm, stream);
-    return push ? launch_one<GS, HAS_K, false, true>(prm, stream) : launch_one<GS, HAS_K, false, false>(prm, stream);
+    if (NT == 1 && prm.M == 1) return push ? launch_one<1, GS, HAS_K, true, true>(prm, stream, taken) : launch_one<1, GS, HAS_K, true, false>(prm, stream, taken);
+    return push ? launch_one<NT, GS, HAS_K, false, true>(prm, stream, taken) : launch_one<NT, GS, HAS_K, false, false>(prm, stream, taken);
 }
 
-cudaError_t launch_any(const GemvParams & prm, bool has_k, cudaStream_t stream) {
+template <int NT>
+cudaError_t launch_any(const GemvParams & prm, bool has_k, cudaStream_t stream, bool * taken) {
     const int gs = prm.G / 64;
     if (has_k) {
-        if (gs == 1) return launch<1, true>(prm, stream);
-        if (gs == 2) return launch<2, true>(prm, stream);
-        return launch<4, true>(prm, stream);
+        if (gs == 1) return launch<NT, 1, true>(prm, stream, taken);
+        if (gs == 2) return launch<NT, 2, true>(prm, stream, taken);
+        return launch<NT, 4, true>(prm, stream, taken);
     }
-    if (gs == 1) return launch<1, false>(prm, stream);
-    if (gs == 2) return launch<2, false>(prm, stream);
-    return launch<4, false>(prm, stream);
+    if (gs == 1) return launch<NT, 1, false>(prm, stream, taken);
+    if (gs == 2) return launch<NT, 2, false>(prm, stream, taken);
+    return launch<NT, 4, false>(prm, stream, taken);
 }
 
 }  // namespace
@@ -389,38 +431,39 @@ cudaError_t rq_launch_gemv(const rq_gemv_job * jobs, int n_jobs, int64_t K, cons
     if (n_jobs < 1 || n_jobs > RQ_MAX_WEIGHTS) return cudaErrorInvalidValue;
     int mt = 0;
     for (int64_t t0 = 0; t0 < M; t0 += mt) {
-        // The stream is read once per pass.  This kernel multiplies up to 8 tokens (one MMA's columns); from 9 tokens on the
-        // tensor-core kernel is the faster one: a decoder layer's four contractions, each launched back to back, take 53 us here
-        // and 58 there at 8 tokens, 59 there at 16 (87 here, with two column tiles) and 108 at 64 (344 in passes of 16).
+        // The stream is read once per pass.  Up to 8 tokens (one MMA's columns) are this kernel's, more than 16 the tensor-core
+        // kernel's (a decoder layer's four contractions, each launched back to back: 108 us at 64 tokens, 344 here in passes of
+        // 16); in between it depends on the sizes.
         mt = (int) (M - t0 < 64 ? M - t0 : 64);
-        if (mt > 8) {
-            rq_gemv_job part[RQ_MAX_WEIGHTS];
+        if (mt <= 16) {
+            GemvParams prm = {};
+            prm.n_jobs = n_jobs;
             for (int i = 0; i < n_jobs; ++i) {
-                part[i] = jobs[i];
-                part[i].y += t0 * jobs[i].ldy;
-                for (int d = 0; d < jobs[i].n_more; ++d) part[i].y_more[d] += t0 * jobs[i].ldy;
+                prm.job[i].w4t = reinterpret_cast<const uint4 *>(jobs[i].w4);
+                prm.job[i].sw = jobs[i].sw;
+                prm.job[i].wk = jobs[i].wk;
+                prm.job[i].y = jobs[i].y + t0 * jobs[i].ldy;
+                prm.job[i].n_more = jobs[i].n_more;
+                for (int d = 0; d < jobs[i].n_more; ++d) prm.job[i].y_more[d] = jobs[i].y_more[d] + t0 * jobs[i].ldy;
+                prm.job[i].ldy = jobs[i].ldy;
+                prm.job[i].N = (int) jobs[i].N;
+                prm.tile_start[i + 1] = prm.tile_start[i] + (int) ((jobs[i].N + 15) / 16);
             }
-            const cudaError_t e = rq_launch_gemm_w4(part, n_jobs, K, a8 + t0 * K, msh + t0 * (K / G), u + t0, mt, G, status, stream);
+            prm.K = (int) K; prm.M = mt; prm.G = G;
+            prm.a8 = a8 + t0 * K; prm.msh = msh + t0 * (K / G); prm.u = u + t0; prm.status = status;
+            const bool has_k = jobs[0].wk != nullptr;
+            bool taken = false;
+            const cudaError_t e = mt <= 8 ? launch_any<1>(prm, has_k, stream, &taken) : launch_any<2>(prm, has_k, stream, &taken);
             if (e != cudaSuccess) return e;
-            continue;
+            if (taken) continue;
         }
-        GemvParams prm = {};
-        prm.n_jobs = n_jobs;
+        rq_gemv_job part[RQ_MAX_WEIGHTS];
         for (int i = 0; i < n_jobs; ++i) {
-            prm.job[i].w4t = reinterpret_cast<const uint4 *>(jobs[i].w4);
-            prm.job[i].sw = jobs[i].sw;
-            prm.job[i].wk = jobs[i].wk;
-            prm.job[i].y = jobs[i].y + t0 * jobs[i].ldy;
-            prm.job[i].n_more = jobs[i].n_more;
-            for (int d = 0; d < jobs[i].n_more; ++d) prm.job[i].y_more[d] = jobs[i].y_more[d] + t0 * jobs[i].ldy;
-            prm.job[i].ldy = jobs[i].ldy;
-            prm.job[i].N = (int) jobs[i].N;
-            prm.tile_start[i + 1] = prm.tile_start[i] + (int) ((jobs[i].N + 15) / 16);
+            part[i] = jobs[i];
+            part[i].y += t0 * jobs[i].ldy;
+            for (int d = 0; d < jobs[i].n_more; ++d) part[i].y_more[d] += t0 * jobs[i].ldy;
         }
-        prm.K = (int) K; prm.M = mt; prm.G = G;
-        prm.a8 = a8 + t0 * K; prm.msh = msh + t0 * (K / G); prm.u = u + t0; prm.status = status;
-        const bool has_k = jobs[0].wk != nullptr;
-        const cudaError_t e = launch_any(prm, has_k, stream);
+        const cudaError_t e = rq_launch_gemm_w4(part, n_jobs, K, a8 + t0 * K, msh + t0 * (K / G), u + t0, mt, G, status, stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
