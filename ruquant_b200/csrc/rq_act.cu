@@ -37,10 +37,15 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-// threads of a prefill CTA: Paley orders up to 72 take two columns per thread (all of them in registers), larger ones one
-constexpr int act_threads(int p) { return p > 1 && p <= 72 ? 128 : 256; }
-constexpr bool act_both(int p) { return p > 44 && p <= 72; }         // 256 threads and a column each where few tokens leave SMs short of warps
-constexpr int act_min_ctas(int p) { return p <= 1 || p > 72 ? 3 : p <= 20 ? 6 : p <= 44 ? 4 : 3; }
+// Threads of a prefill CTA.  Paley orders up to 60 take two columns per thread in registers (spilled: 8 bytes with order 44, 16 with
+// 60), and where few tokens leave SMs short of warps 256 threads with one column each.  Larger orders: 256 threads only.  Two
+// columns of 68 or 72 inputs do not fit the registers (288 and 400 bytes spilled), and between a GEMM and the next that form is
+// the slower one at every number of tokens: the 17408 x 5120 node with 700, 1024 and 4096 tokens 173, 234 and 691 us, 143, 208 and
+// 687 with 256 threads.
+constexpr int act_threads(int p) { return p > 1 && p <= 60 ? 128 : 256; }
+constexpr bool act_both(int p) { return act_threads(p) == 128; }
+// CTAs an SM that the registers have to admit: three of 256 threads (80 registers), or of 128 threads what leaves the columns room
+constexpr int act_min_ctas(int p, int threads) { return threads == 256 || p > 44 ? 3 : p <= 20 ? 6 : 4; }
 // threads of a cluster CTA: every phase is latency, so as many warps as the Paley stage's registers allow (it reads its
 // P inputs once each, the compiler keeps them at about 55-64 registers)
 constexpr int cluster_threads(int p) { return p <= 72 ? 1024 : 512; }
@@ -65,7 +70,7 @@ struct ActParams {
 // P > 1: Paley order (compile time); P == 1: no Paley stage (plain W4A4, or a power-of-two rotation).
 // shared memory: [K floats row][P*P floats sign table]
 template <int P, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P) : 1) rq_act_kernel(const ActParams prm) {
+__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THREADS) : 1) rq_act_kernel(const ActParams prm) {
     extern __shared__ __align__(16) float buf[];
     __shared__ float g_lo[512], g_hi[512];
     __shared__ float red[THREADS / 32];
@@ -415,8 +420,7 @@ cudaError_t launch(const ActParams & prm, int64_t M, cudaStream_t stream) {
     // few tokens and a cheap Paley stage: one big CTA per token keeps every phase short
     static const int wide = rq_env_int("RQ_TUNE_ACT_WIDE", 1);
     if (P <= 20 && M <= 64 && wide) return launch_ex(rq_act_kernel<(P <= 20 ? P : 1), 1024>, dim3((unsigned) M), dim3(1024), smem, 1, stream, prm);
-    // up to four tokens an SM the phases are latency: twice the warps (512 tokens of 17408: 47 us, 51 with 128 threads; 4096: 277, 268)
-    if (act_both(P) && M <= 4 * sms[dev]) return launch_ex(rq_act_kernel<(act_both(P) ? P : 1), 256>, dim3((unsigned) M), dim3(256), smem_row, 1, stream, prm);
+    if (act_both(P) && rq_act_256(P, K, M, sms[dev])) return launch_ex(rq_act_kernel<(act_both(P) ? P : 1), 256>, dim3((unsigned) M), dim3(256), smem_row, 1, stream, prm);
     return launch_ex(rq_act_kernel<P, act_threads(P)>, dim3((unsigned) M), dim3(act_threads(P)), smem_row, 1, stream, prm);
 }
 

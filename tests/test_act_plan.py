@@ -30,3 +30,17 @@ def test_cluster_width(tmp_path, asked):
     for units, M, c in rows:
         ok = [w for w in (1, 2, 4, 8) if w == 1 or (w <= asked and units >= 2 * w and M <= fits[w])]
         assert c == max(ok), (asked, units, M)
+
+
+def test_threads_of_a_prefill_cta(tmp_path):
+    """256 threads while the tokens are few, never again once 128 have been taken; at the sizes both forms were measured at"""
+    out = run(tmp_path, """
+    const int p[6] = { 12, 12, 20, 12, 44, 60 }, K[6] = { 768, 3072, 5120, 6144, 11264, 15360 };
+    for (int i = 0; i < 6; ++i) {
+        for (int M = 1; M < 2000; ++M) putchar(rq_act_256(p[i], K[i], M, 148) ? '1' : '0');
+        putchar('\\n');
+    }""")
+    rows = out.split()
+    last = [row.rfind("1") + 1 for row in rows]
+    assert all(row == "1" * n + "0" * (1999 - n) for row, n in zip(rows, last))
+    assert last == [444, 444, 592, 592, 444, 444]
