@@ -188,21 +188,31 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THRE
     if (tid == 0) prm.u[t] = unit;
     RQ_STAMP(tid == 0);                                     // 4: ranges reduced
 
-    // the groups' constants once per group (two divisions), in place of their ranges
+    // The groups' constants (two divisions).  Where a thread has several words: once per group, in place of the ranges.  With one
+    // or two each the pass and its barrier cost more than the divisions they save (150 tokens of 3072 4.2 us, 4.1; 8 of 768 3.5,
+    // 3.4; 6144 in groups of 128 at one token 6.4, 6.3): every lane makes its own.
     int32_t * mrow = prm.msh + (int64_t) t * (K / prm.G);
-    for (int g = tid; g < K / prm.G; g += nt) {
-        float mf, inv, zf;
-        group_constants(g_lo[g], g_hi[g], R, unit, mf, inv, zf);
-        mrow[g] = prm.fmt == RQ_FMT_E4M3 ? multiplier_word<true>(mf) : multiplier_word<false>(mf);
-        g_lo[g] = inv;
-        g_hi[g] = zf;
+    const bool once = nwords > 2 * nt;
+    if (once) {
+        for (int g = tid; g < K / prm.G; g += nt) {
+            float mf, inv, zf;
+            group_constants(g_lo[g], g_hi[g], R, unit, mf, inv, zf);
+            mrow[g] = prm.fmt == RQ_FMT_E4M3 ? multiplier_word<true>(mf) : multiplier_word<false>(mf);
+            g_lo[g] = inv;
+            g_hi[g] = zf;
+        }
+        __syncthreads();
     }
-    __syncthreads();
     int8_t * arow = prm.a8 + (int64_t) t * K + run_offset(l);
     auto store_codes = [&](auto f8) {
         constexpr bool F8 = decltype(f8)::value;
         for (int w = tid; w < nwords; w += nt) {
-            const float inv = g_lo[w >> llpg], zf = g_hi[w >> llpg];
+            float inv = g_lo[w >> llpg], zf = g_hi[w >> llpg];
+            if (!once) {
+                float mf;
+                group_constants(g_lo[w >> llpg], g_hi[w >> llpg], R, unit, mf, inv, zf);
+                if ((w & (lpg - 1)) == 0) mrow[w >> llpg] = multiplier_word<F8>(mf);
+            }
             const uint32_t ca = encode4<F8>(buf4[(w >> 3) * 16 + off_a], inv, zf), cb = encode4<F8>(buf4[(w >> 3) * 16 + off_b], inv, zf);
             *reinterpret_cast<uint2 *>(arow + (w >> 3) * 64) = run_codes(l, ca, cb);
         }
