@@ -292,9 +292,11 @@ __device__ __forceinline__ void transform_runs_inplace(float * buf, int count, i
 __device__ __forceinline__ void fwht_resident(float * buf, int len, int m, int tid, int nt, int bar = 0) {
     const int warp = tid >> 5, nwarps = nt >> 5, lane = tid & 31;
     // register runs of up to 1024 values, shorter (down to 256) where there would be fewer of them than warps (4096 tokens of
-    // 4096: 85 us with the four runs of 1024 on eight warps, 65 with 16 of 256 and two passes over shared memory)
+    // 4096: 85 us with the four runs of 1024 on eight warps, 65 with 16 of 256 and two passes over shared memory); but whole chunks
+    // stay whole where eight warps have one, since splitting those adds a pass (a token of 6144 on 32 warps: 12 runs of 512 6.0 us,
+    // 24 of 256 6.3)
     int run = m < 1024 ? m : 1024;
-    while (run > 256 && len / run < nwarps) run >>= 1;
+    while (run > 256 && len / run < nwarps && (run < m || len / run < 8)) run >>= 1;
     switch (run) {
         case 32:   if (m > 1) transform_runs_inplace<1>(buf, len / 32, warp, nwarps, lane); break;
         case 64:   transform_runs_inplace<2>(buf, len / 64, warp, nwarps, lane); break;
