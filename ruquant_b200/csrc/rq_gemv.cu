@@ -91,6 +91,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// CTAs an SM that the compiler is asked to leave registers for; 0: its own choice.
+//   two tiles, groups of 256, multipliers   left alone 132 registers, one CTA: 9 tokens of 5120 x 4096 7.2 us, 5.2 with two
+//   one token, groups of 128                left alone 72 registers, three CTAs: 17408 x 8192 15.7 us, 11.9 with two
+//   several, groups of 128, multipliers     left alone 56 registers: 8 tokens of 17408 x 17408 46 us, 37 with 72
+constexpr int gemv_ctas_asked(int nt, int gs, bool has_k, bool one) {
+    if (nt == 2) return gs == 4 && has_k ? 2 : 0;
+    if (gs == 2 && one && !has_k) return 2;
+    return gs == 2 && !one && has_k ? 3 : 0;
+}
+
 // Persistent CTAs, three per SM, each walking tiles of 16 weight rows (tile = blockIdx.x, += gridDim.x).  The producer
 // warp streams the tiles' K/64 * 512 bytes back to back into a shared-memory ring with bulk copies (it starts at once:
 // the weights do not depend on the preceding kernel, and it never drains between tiles); the consumer warps take the
@@ -98,7 +108,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // NT: token tiles of 8 (1 or 2).  GS: 64-input steps per activation group (1, 2, 4).  HAS_K: weight multipliers.
 // ONE: M == 1 (only token 0 is folded and stored).  PUSH: outputs also go to the jobs' further destinations.
 template <int NT, int GS, bool HAS_K, bool ONE, bool PUSH>
-__global__ void __launch_bounds__((CONSUMERS + 1) * 32) rq_gemv_mma_kernel(const GemvParams prm) {
+__global__ void __launch_bounds__((CONSUMERS + 1) * 32, gemv_ctas_asked(NT, GS, HAS_K, ONE)) rq_gemv_mma_kernel(const GemvParams prm) {
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ uint64_t full[STAGES], empty[STAGES];
     __shared__ int abort_word;
@@ -386,7 +396,7 @@ cudaError_t launch_one(const GemvParams & prm, cudaStream_t stream, bool * taken
     const cudaError_t e = resident_ctas<NT, GS, HAS_K, ONE, PUSH>(&resident);
     if (e != cudaSuccess) return e;
     const int tiles = prm.tile_start[prm.n_jobs];
-    *taken = NT == 1 || rq_gemv_takes_16(prm.K, tiles, resident, prm.M);
+    *taken = NT == 1 || rq_gemv_takes_16(prm.K, tiles, resident, prm.M, prm.G, HAS_K);
     if (!*taken) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     // (an evenly divided grid -- every CTA the same number of tiles -- measured slower: 3.79 against 3.68 ms per pass)

@@ -14,9 +14,14 @@
 //   two rounds    1024 x 8192 4.4, 6.1; 4096 x 8192 8.4, 9.0; 5120 x 8192 from L2 9.0, 9.4; 256 x 8192 from L2 4.0, 3.2 (a single
 //                 slice of K: no cluster, nothing to hand over)
 //   three rounds  1024 x 12288 6.2, 4.9
-inline bool rq_gemv_takes_16(int64_t K, int64_t tiles, int64_t ctas, int64_t M) {
+// Groups of 128 and 256 inputs need a half and a quarter of the folds: 6144 x 4096 in groups of 256 5.5, 7.5; 5120 x 8192 7.8, 8.7;
+// 11264 x 2048 with 16 tokens in groups of 128 6.6, 7.7.  Weight multipliers cost the tensor-core kernel more.
+inline bool rq_gemv_takes_16(int64_t K, int64_t tiles, int64_t ctas, int64_t M, int group, bool has_k) {
+    const int64_t any_m = group == 64 ? 4096 : 6144;      // inputs up to which the number of tokens makes no difference
     if (tiles > 2 * ctas) return false;
-    if (tiles > ctas) return K > 256 && K <= 4096;
-    if (K <= 4096) return true;
-    return K * M <= (tiles >= 128 ? 96 : tiles >= 64 ? 64 : 0) * 1024;
+    if (tiles > ctas) return K > 256 && K <= any_m;
+    if (K <= any_m) return true;
+    if (tiles < 64) return false;
+    const int64_t many = group == 64 ? 96 : group == 128 ? 192 : 144, few = group == 64 ? (has_k ? 80 : 64) : group == 128 ? 112 : 80;
+    return K * M <= 1024 * (tiles >= 128 ? many : few);
 }

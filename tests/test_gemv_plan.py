@@ -17,12 +17,12 @@ MEASURED = [(256, 16, 288, 16, GEMV), (1024, 4096, 288, 9, GEMV), (1024, 4096, 1
 @pytest.fixture(scope="module")
 def takes(tmp_path_factory):
     d = tmp_path_factory.mktemp("gemv")
-    (d / "p.cpp").write_text('#include <stdio.h>\n#include "rq_gemv_plan.h"\nint main() { long long k, t, c, m;\n'
-                             'while (scanf("%lld %lld %lld %lld", &k, &t, &c, &m) == 4) printf("%d\\n", (int) rq_gemv_takes_16(k, t, c, m)); return 0; }\n')
+    (d / "p.cpp").write_text('#include <stdio.h>\n#include "rq_gemv_plan.h"\nint main() { long long k, t, c, m, g;\n'
+                             'while (scanf("%lld %lld %lld %lld %lld", &k, &t, &c, &m, &g) == 5) printf("%d\\n", (int) rq_gemv_takes_16(k, t, c, m, (int) g, c == 140)); return 0; }\n')
     subprocess.check_call(["g++", "-std=c++17", "-I", CSRC, str(d / "p.cpp"), "-o", str(d / "p")])
 
-    def ask(points):
-        text = "\n".join("%d %d %d %d" % (K, (N + 15) // 16, ctas, M) for K, N, ctas, M in points)
+    def ask(points, group=64):
+        text = "\n".join("%d %d %d %d %d" % (K, (N + 15) // 16, ctas, M, group) for K, N, ctas, M in points)
         return [int(v) for v in subprocess.run([str(d / "p")], input=text, capture_output=True, text=True, check=True).stdout.split()]
 
     return ask
@@ -30,6 +30,8 @@ def takes(tmp_path_factory):
 
 def test_where_it_was_measured(takes):
     assert takes([p[:4] for p in MEASURED]) == [p[4] for p in MEASURED]
+    assert takes([(6144, 4096, 288, 16), (5120, 8192, 288, 16), (8192, 4096, 288, 16), (17408, 2048, 140, 9), (17408, 17408, 288, 9)], 256) == [
+        GEMV, GEMV, GEMV, TENSOR_CORES, TENSOR_CORES]
 
 
 def test_more_tokens_inputs_or_rows_never_come_back_to_the_gemv(takes):
