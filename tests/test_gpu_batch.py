@@ -70,3 +70,69 @@ def test_three_weights_and_token_passes(rq, port):
         rq.device_status(work, K, M)
         for wb, y, N in zip(wbs, ys, rows):
             assert_bits(y.cpu().numpy(), port.mul_mat(wb, 45, K, x), "M=%d N=%d" % (M, N))
+
+
+GROUPS = [(64, 0), (128, 0), (256, 0), (64, 64), (64, 256), (128, 256), (256, 256)]
+DISTINCT = 160
+
+
+def tiled_weight(rq, port, type_, N, M, K, wgroup, seed):
+    """N rows out of DISTINCT that repeat: the oracle multiplies those, the copies have to agree with them"""
+    wb, x = case(port, type_, DISTINCT, M, K, wgroup, seed)
+    blocks = dev(wb).repeat((N + DISTINCT - 1) // DISTINCT, 1)[:N].contiguous()
+    return rq.Weight(blocks.view(-1), type_, K, N=N, layouts=rq.PREPACK_DECODE), wb, x
+
+
+def check_tiled(port, wb, type_, K, x, y, group, what):
+    assert_bits(y[:, :DISTINCT].cpu().numpy(), port.mul_mat(wb, type_, K, x, group=group), what)
+    whole = y.shape[1] // DISTINCT * DISTINCT
+    bits = y.contiguous().view(torch.int32)
+    assert (bits[:, :whole].view(y.shape[0], -1, DISTINCT) == bits[:, None, :DISTINCT]).all(), what
+    assert (bits[:, whole:] == bits[:, :y.shape[1] - whole]).all(), what
+
+
+@pytest.mark.parametrize("M", [16, 30, 47, 64])
+@pytest.mark.parametrize("group,wgroup", GROUPS)
+def test_many_tiles_a_cta_in_every_mode(rq, port, M, group, wgroup):
+    """more row tiles than CTAs (K not split) and 16 slices of K a tile: every ring, the accumulator sets and the multiplier slots
+    wrap several times, for each tile width, activation group and multiplier mode"""
+    K, N = 4096, 40000
+    w, wb, x = tiled_weight(rq, port, 44, N, M, K, wgroup, 13)
+    work = rq.new_workspace(K, M)
+    y = rq.mul_mat(w, dev(x), act_group=group, workspace=work)
+    torch.cuda.synchronize()
+    rq.device_status(work, K, M)
+    check_tiled(port, wb, 44, K, x, y, group, "M=%d group=%d wgroup=%d" % (M, group, wgroup))
+
+
+@pytest.mark.parametrize("M", [2, 8, 9, 16])
+@pytest.mark.parametrize("group,wgroup", GROUPS)
+@pytest.mark.parametrize("N", [1000, 8200])
+def test_gemv_tiles(rq, port, M, group, wgroup, N):
+    """the GEMV with one and two tiles of 8 tokens: one and several rounds of row tiles a CTA, a ragged last tile"""
+    K = 1024
+    w, wb, x = tiled_weight(rq, port, 44, N, M, K, wgroup, 17)
+    work = rq.new_workspace(K, M)
+    y = rq.mul_mat(w, dev(x), act_group=group, workspace=work)
+    torch.cuda.synchronize()
+    rq.device_status(work, K, M)
+    check_tiled(port, wb, 44, K, x, y, group, "M=%d N=%d group=%d wgroup=%d" % (M, N, group, wgroup))
+
+
+@pytest.mark.parametrize("wgroup", [0, 64])
+@pytest.mark.parametrize("M,N,K", [(12, 328, 1024), (16, 328, 5120), (47, 328, 5120), (64, 328, 5120), (16, 20008, 1024), (47, 20008, 1024), (64, 20008, 1024)])
+def test_push(rq, port, M, N, K, wgroup):
+    """outputs into two destinations, the second 4 bytes off a 16-byte boundary and both wider than the weight: from the GEMV's
+    two tiles (12 tokens), from clusters that split K (328 rows) and from CTAs that walk whole tiles (20008 rows)"""
+    w, wb, x = tiled_weight(rq, port, 44, N, M, K, wgroup, 19)
+    ld = N + 8
+    a = torch.full((M, ld), -1.0, device="cuda")
+    b = torch.full((M * ld + 1,), -1.0, device="cuda")
+    work = rq.new_workspace(K, M)
+    rq.mul_mat_push([w], dev(x), [[a.data_ptr()], [b.data_ptr() + 4]], [ld], workspace=work)
+    torch.cuda.synchronize()
+    rq.device_status(work, K, M)
+    for got in (a, b[1:].view(M, ld)):
+        check_tiled(port, wb, 44, K, x, got[:, :N], 64, "push M=%d N=%d wgroup=%d" % (M, N, wgroup))
+        assert (got[:, N:] == -1.0).all()
+    assert float(b[0]) == -1.0
