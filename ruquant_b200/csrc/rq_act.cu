@@ -99,8 +99,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THRE
         // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
         bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid, prm.status);
     } else {
-        copy_row(buf, xrow, K, tid, nt);           // (a rotation without a workspace has nowhere to report a wait that ran out)
-        __syncthreads();
+        load_row_surely(buf, xrow, K, &row_bar, tid, nt);      // (a rotation without a workspace has nowhere to report a wait that ran out)
     }
     if (prm.n_rot > 0) {
         fwht_resident(buf, K, prm.m, tid, nt);

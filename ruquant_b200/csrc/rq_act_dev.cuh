@@ -339,24 +339,34 @@ __device__ __forceinline__ void await_row(uint32_t bar, int32_t * status, long l
 // One bulk asynchronous copy of a row (bytes a multiple of 16, both ends 16-byte aligned) into shared memory, issued by
 // one thread, awaited by all: a single trip to memory for the whole row, where per-run loads expose one trip per round of
 // runs a warp takes.
+__device__ __forceinline__ void issue_row(float * dst, const float * src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void bulk_load_row(float * dst, const float * src, uint32_t bytes, uint64_t * bar, int tid, int32_t * status) {
     const uint32_t b = (uint32_t) __cvta_generic_to_shared(bar);
-    if (tid == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(bytes) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"(bytes), "r"(b) : "memory");
-    }
+    if (tid == 0) issue_row(dst, src, bytes, b);
     await_row(b, status);
 }
 
-// A row by 16-byte asynchronous copies of every thread, all of them in flight at once and waited for as loads are: no barrier
-// word, nothing that could run out.  A thread sees the pieces tid, tid + nt, ... that it copied itself, the others behind a
-// CTA barrier.
-__device__ __forceinline__ void copy_row(float * dst, const float * src, int len, int tid, int nt) {
-    const uint32_t d = (uint32_t) __cvta_generic_to_shared(dst);
-    for (int i = tid; i < len / 4; i += nt)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(d + (uint32_t) i * 16u), "l"(src + 4 * i) : "memory");
-    asm volatile("cp.async.wait_all;" ::: "memory");
+// The wait of callers that have no error word: if it runs out for any thread, the row is copied again by asynchronous 16-byte
+// copies of all threads, which are waited for as loads are and cannot run out (a bulk copy that lands late writes the same
+// bytes).  Ends with a CTA barrier.
+__device__ __forceinline__ void await_row_or_copy(uint32_t bar, float * dst, const float * src, int len, int tid, int nt, long long cycles = 2000000000ll) {
+    if (__syncthreads_or(!row_landed(bar, cycles))) {
+        row_landed(bar, cycles);
+        const uint32_t d = (uint32_t) __cvta_generic_to_shared(dst);
+        for (int i = tid; i < len / 4; i += nt)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(d + (uint32_t) i * 16u), "l"(src + 4 * i) : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+}
+__device__ __forceinline__ void load_row_surely(float * dst, const float * src, int len, uint64_t * bar, int tid, int nt) {
+    const uint32_t b = (uint32_t) __cvta_generic_to_shared(bar);
+    if (tid == 0) issue_row(dst, src, (uint32_t) len * 4u, b);
+    await_row_or_copy(b, dst, src, len, tid, nt);
 }
 
 // A buffer of `len` floats made of whole chunks of m: loaded from global memory and Sylvester-transformed chunk by

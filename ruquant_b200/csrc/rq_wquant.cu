@@ -125,14 +125,19 @@ __global__ void __launch_bounds__(WROW_THREADS) rq_wrow_kernel(const float * __r
     __shared__ int red_i[WROW_THREADS / 32];
     __shared__ float win_s;
     __shared__ unsigned contested_s;
+    __shared__ uint64_t row_bar;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t row = blockIdx.x;
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((uint32_t) __cvta_generic_to_shared(&row_bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
     const float * xr = x + row * ldx;
 
-    // (not by a bulk copy, whose wait may run out: a conversion has nowhere to report that)
-    rq_act_dev::copy_row(xs, xr, K, tid, WROW_THREADS);
+    rq_act_dev::load_row_surely(xs, xr, K, &row_bar, tid, WROW_THREADS);
 
-    float amax = 0.0f;                            // (of the pieces this thread copied: no barrier yet)
+    float amax = 0.0f;
     for (int i = tid; i < K / 4; i += WROW_THREADS) {
         const float4 q = reinterpret_cast<const float4 *>(xs)[i];
         amax = fmaxf(fmaxf(fmaxf(amax, fabsf(q.x)), fmaxf(fabsf(q.y), fabsf(q.z))), fabsf(q.w));
