@@ -244,7 +244,8 @@ def mul_mat(weights, x, out=None, clip=None, act_group=None, path=PATH_AUTO, wor
         ws = workspace
         if ws is None:
             # used by this call alone, on the stream that its status block is zeroed on: nothing to wait for
-            ws = _empty_on(stream, workspace_bytes(K, M), device)
+            nbytes = L.rq_w4a4_workspace_bytes(K, M)
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=device) if stream is None else _empty_on(stream, nbytes, device)
             _check(L.rq_w4a4_workspace_init(ws.data_ptr(), K, M, handle), "rq_w4a4_workspace_init")
         _check(L.rq_w4a4_mul_mat(descs, n_w, x.data_ptr(), x.stride(0), M, ys, ldy, clip, act_group, path, ws.data_ptr(), ws.numel(),
                                  handle), "rq_w4a4_mul_mat")
