@@ -895,16 +895,19 @@ cudaError_t rq_launch_gemm_tc(const rq_gemm_job * jobs, int n_jobs, int fmt, int
     // Weight rows per tile: the widest tile costs least per row (the 128 x 64 token operand and every hand-over are shared by
     // more columns), but a launch takes whole rounds of one unit per SM, and one of 5120 rows and 512 tokens has 80 units of
     // 256 rows for 148 SMs.  The narrower tile is taken where it saves more rounds than its rounds are dearer per row.  Time of a
-    // round measured with K = 17408: 82, 70, 64 and 57 us for 256, 192, 160 and 128 rows of fp8 operands, and in proportion to
-    // 105, 75, 68 and 54 for integer ones (K = 11264: the integer fold, two instructions per sum, weighs more).
+    // round with 256, 192, 160 and 128 rows, fp8 operands, the last of three full rounds, us: K = 4096 23.5, 20.0, 18.2, 16.3; 11264
+    // 54, 46, 41, 38; 17408 84, 76, 62, 56; in groups of 256 11264 41, 33, 31, 28.  Integer operands in groups of 256: 11264 44, 34, 32,
+    // 29, in about the same proportion; in groups of 64, where their fold of two instructions per sum weighs more, narrow tiles are
+    // cheaper: 4096 37, 27, 25, 22; 11264 97, 68, 60, 55; 17408 159, 111, 97, 84.
     static const int rows_nq[4] = { 8, 6, 5, 4 }, cost[2][4] = { { 105, 75, 68, 54 }, { 82, 70, 64, 57 } };
+    const bool even = f8 || G > 64;
     int nq = 8, units = 0;
     long best = 0;
     for (int c = 0; c < (push ? 1 : 4); ++c) {
         int tiles = 0;
         for (int i = 0; i < n_jobs; ++i) tiles += (int) ((jobs[i].N + 32 * rows_nq[c] - 1) / (32 * rows_nq[c]));
         const int n = tiles * m_tiles;
-        const long time = (long) ((n + sms - 1) / sms) * cost[f8][c];
+        const long time = (long) ((n + sms - 1) / sms) * cost[even][c];
         if (c == 0 || time < best) { best = time; nq = rows_nq[c]; units = n; }
     }
 
