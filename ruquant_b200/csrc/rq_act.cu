@@ -95,12 +95,8 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THRE
     RQ_STAMP(tid == 0);                                     // 1: after the wait
 
     const float * xrow = prm.x + (int64_t) t * prm.ldx;
-    if (prm.status != nullptr) {
-        // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
-        bulk_load_row(buf, xrow, (uint32_t) K * 4u, &row_bar, tid, prm.status);
-    } else {
-        load_row_surely(buf, xrow, K, &row_bar, tid, nt);      // (a rotation without a workspace has nowhere to report a wait that ran out)
-    }
+    // the row arrives in one bulk copy (thousands of tokens: what counts is trips to memory per token, and this is one)
+    bulk_load_row(buf, xrow, K, &row_bar, tid, nt, prm.status);
     if (prm.n_rot > 0) {
         fwht_resident(buf, K, prm.m, tid, nt);
         RQ_STAMP(tid == 0);                                 // 2: chunks transformed
@@ -187,12 +183,12 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THRE
     if (tid == 0) prm.u[t] = unit;
     RQ_STAMP(tid == 0);                                     // 4: ranges reduced
 
-    // The groups' constants (two divisions).  Where a thread has several words: once per group, in place of the ranges.  With one
-    // or two each the pass and its barrier cost more than the divisions they save (150 tokens of 3072 4.2 us, 4.1; 8 of 768 3.5,
-    // 3.4; 6144 in groups of 128 at one token 6.4, 6.3): every lane makes its own.
+    // The groups' constants (two divisions): once per group, in place of the ranges.  The 1024 threads of a small call have a word or
+    // two each, and the pass and its barrier would cost more than the divisions they save (768 inputs 3.5 us a launch, 3.4; 6144
+    // in groups of 128 at one token 6.4, 6.3): there every lane makes its own.
+    constexpr bool ONCE = THREADS <= 256;
     int32_t * mrow = prm.msh + (int64_t) t * (K / prm.G);
-    const bool once = nwords > 2 * nt;
-    if (once) {
+    if constexpr (ONCE) {
         for (int g = tid; g < K / prm.G; g += nt) {
             float mf, inv, zf;
             group_constants(g_lo[g], g_hi[g], R, unit, mf, inv, zf);
@@ -207,7 +203,7 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 256 ? act_min_ctas(P, THRE
         constexpr bool F8 = decltype(f8)::value;
         for (int w = tid; w < nwords; w += nt) {
             float inv = g_lo[w >> llpg], zf = g_hi[w >> llpg];
-            if (!once) {
+            if constexpr (!ONCE) {
                 float mf;
                 group_constants(g_lo[w >> llpg], g_hi[w >> llpg], R, unit, mf, inv, zf);
                 if ((w & (lpg - 1)) == 0) mrow[w >> llpg] = multiplier_word<F8>(mf);

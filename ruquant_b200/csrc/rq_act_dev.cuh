@@ -327,34 +327,22 @@ __device__ __forceinline__ bool row_landed(uint32_t bar, long long cycles) {
         if ((i & 63u) == 63u && clock64() - t0 > cycles) return false;
     }
 }
-// The wait for it, by every thread of the CTA.  A thread whose wait runs out (about a second) sets the error word and waits once
-// more, so that the CTA does not end under a copy that is still in flight; then it goes on with what the buffer holds.  No thread
-// leaves: others may have seen the copy land, and the barriers and shuffles that follow are for all of them.  (Whatever the
-// floats, codes are bytes and every index is in range; the error word says that the results are not to be used.)
-__device__ __forceinline__ void await_row(uint32_t bar, int32_t * status, long long cycles = 2000000000ll) {
-    if (row_landed(bar, cycles)) return;
-    atomicExch(status, 1);
-    row_landed(bar, cycles);
-}
-// One bulk asynchronous copy of a row (bytes a multiple of 16, both ends 16-byte aligned) into shared memory, issued by
-// one thread, awaited by all: a single trip to memory for the whole row, where per-run loads expose one trip per round of
-// runs a warp takes.
-__device__ __forceinline__ void issue_row(float * dst, const float * src, uint32_t bytes, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void bulk_load_row(float * dst, const float * src, uint32_t bytes, uint64_t * bar, int tid, int32_t * status) {
-    const uint32_t b = (uint32_t) __cvta_generic_to_shared(bar);
-    if (tid == 0) issue_row(dst, src, bytes, b);
-    await_row(b, status);
-}
-
-// The wait of callers that have no error word: if it runs out for any thread, the row is copied again by asynchronous 16-byte
-// copies of all threads, which are waited for as loads are and cannot run out (a bulk copy that lands late writes the same
-// bytes).  Ends with a CTA barrier.
-__device__ __forceinline__ void await_row_or_copy(uint32_t bar, float * dst, const float * src, int len, int tid, int nt, long long cycles = 2000000000ll) {
-    if (__syncthreads_or(!row_landed(bar, cycles))) {
+// The wait for it, by every thread of the CTA.  If it runs out (about a second) a caller with an error word has it set, and the
+// thread waits once more, so that the CTA does not end under a copy that is still in flight; then it goes on with what the buffer
+// holds.  No thread leaves: others may have seen the copy land, and the barriers and shuffles that follow are for all of them.
+// (Whatever the floats, codes are bytes and every index is in range; the error word says that the results are not to be used.)
+// Without an error word the row has to be there: if the wait runs out for any thread, all of them copy the row again by
+// asynchronous 16-byte copies, which are waited for as loads are and cannot run out (a bulk copy that lands late writes the
+// same bytes).
+__device__ __forceinline__ void await_row(uint32_t bar, float * dst, const float * src, int len, int tid, int nt, int32_t * status,
+                                          long long cycles = 2000000000ll) {
+    const bool late = !row_landed(bar, cycles);
+    if (status != nullptr) {
+        if (late) {
+            atomicExch(status, 1);
+            row_landed(bar, cycles);
+        }
+    } else if (__syncthreads_or(late)) {
         row_landed(bar, cycles);
         const uint32_t d = (uint32_t) __cvta_generic_to_shared(dst);
         for (int i = tid; i < len / 4; i += nt)
@@ -363,10 +351,16 @@ __device__ __forceinline__ void await_row_or_copy(uint32_t bar, float * dst, con
         __syncthreads();
     }
 }
-__device__ __forceinline__ void load_row_surely(float * dst, const float * src, int len, uint64_t * bar, int tid, int nt) {
+// A row by one bulk asynchronous copy (len a multiple of 4, both ends 16-byte aligned) into shared memory, issued by one thread,
+// awaited by all: a single trip to memory for the whole row, where per-run loads expose one trip per round of runs a warp takes.
+__device__ __forceinline__ void bulk_load_row(float * dst, const float * src, int len, uint64_t * bar, int tid, int nt, int32_t * status) {
     const uint32_t b = (uint32_t) __cvta_generic_to_shared(bar);
-    if (tid == 0) issue_row(dst, src, (uint32_t) len * 4u, b);
-    await_row_or_copy(b, dst, src, len, tid, nt);
+    if (tid == 0) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"((uint32_t) len * 4u) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"((uint32_t) len * 4u), "r"(b) : "memory");
+    }
+    await_row(b, dst, src, len, tid, nt, status);
 }
 
 // A buffer of `len` floats made of whole chunks of m: loaded from global memory and Sylvester-transformed chunk by

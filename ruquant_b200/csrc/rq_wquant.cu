@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(WROW_THREADS) rq_wrow_kernel(const float * __r
     __syncthreads();
     const float * xr = x + row * ldx;
 
-    rq_act_dev::load_row_surely(xs, xr, K, &row_bar, tid, WROW_THREADS);
+    rq_act_dev::bulk_load_row(xs, xr, K, &row_bar, tid, WROW_THREADS, nullptr);      // (nowhere to report to: copied again if it does not land)
 
     float amax = 0.0f;
     for (int i = tid; i < K / 4; i += WROW_THREADS) {

@@ -25,7 +25,7 @@ __global__ void probe(int32_t * status, int32_t * seen, long long cycles, int ar
     }
     __syncthreads();
     if (threadIdx.x == 0 && arrive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(b) : "memory");
-    rq_act_dev::await_row(b, status, cycles);
+    rq_act_dev::await_row(b, nullptr, nullptr, 0, threadIdx.x, blockDim.x, status, cycles);
     atomicAdd(&n, 1);
     __syncthreads();
     seen[threadIdx.x] = n;
@@ -42,8 +42,8 @@ __global__ void surely(const float * src, float * out, int len, long long cycles
     }
     __syncthreads();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (issue) rq_act_dev::load_row_surely(buf, src, len, &bar, threadIdx.x, blockDim.x);
-    else rq_act_dev::await_row_or_copy(b, buf, src, len, threadIdx.x, blockDim.x, cycles);
+    if (issue) rq_act_dev::bulk_load_row(buf, src, len, &bar, threadIdx.x, blockDim.x, nullptr);
+    else rq_act_dev::await_row(b, buf, src, len, threadIdx.x, blockDim.x, nullptr, cycles);
     for (int i = threadIdx.x; i < len; i += blockDim.x) out[i] = buf[len - 1 - i];
 }
 extern "C" __attribute__((visibility("default"))) int run_surely(const float * src, float * out, int len, int threads, long long cycles, int issue) {

@@ -13,13 +13,19 @@ def code(name):
 
 def test_weight_conversion_has_no_way_out():
     text = code("rq_wquant.cu")
-    assert text.count("load_row_surely(") == 1 and not re.search(r"bulk_load_row|try_wait|row_landed|clock64", text)
-    kernels = text[:text.index("cudaError_t rq_launch_wquant")]
-    assert not re.search(r"\breturn;", kernels)
+    assert len(re.findall(r"bulk_load_row\([^;]*, nullptr\);", text)) == 1
+    assert not re.search(r"try_wait|row_landed|await_row|clock64", text)
+    assert not re.search(r"\breturn;", text[:text.index("cudaError_t rq_launch_wquant")])
 
 
-def test_rotation_without_a_status_word_has_none_either():
+def test_rotation_has_none_either():
     text = code("rq_act.cu")
-    at = text.index("bulk_load_row(")
-    assert text.count("bulk_load_row(") == 1 and "if (prm.status != nullptr) {" in text[at - 60:at]
-    assert re.match(r"bulk_load_row\([^;]*;\s*\} else \{\s*load_row_surely\(", text[at:])
+    assert len(re.findall(r"^ {4}bulk_load_row\([^;]*, prm\.status\);", text, re.M)) == 1
+    body = text[text.index("rq_act_kernel(const ActParams prm)"):]
+    assert not re.search(r"\breturn;", body[:body.index("if (prm.a8 == nullptr) return;")])
+
+
+def test_the_wait_without_a_status_word_ends_with_the_row():
+    text = code("rq_act_dev.cuh")
+    wait = text[text.index("void await_row("):text.index("void bulk_load_row(")]
+    assert re.search(r"\} else if \(__syncthreads_or\(late\)\) \{.*cp\.async\.wait_all", wait, re.S) and "return" not in wait
