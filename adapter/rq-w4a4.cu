@@ -92,8 +92,9 @@ void ggml_cuda_mul_mat_rq_w4a4(ggml_backend_cuda_context & ctx, const ggml_tenso
 }
 
 // The reference's predicate (patch:2350-2368) with its kernel-specific part replaced: there "both run the skinny kernel",
-// here "both have been prepared" (which also implies both were seen outside a capture).  The width limit of 16 tokens is
-// kept: wider inputs gain nothing from one launch over all rows.
+// here "both have been prepared" (which also implies both were seen outside a capture).  The reference's width limit of 16
+// tokens is kept, so that the graph is cut into the same nodes; the library itself takes up to three weights in one launch at any
+// width, and wider inputs, which would then share the quantizer too, do without that here.
 bool ggml_cuda_rq_w4a4_can_fuse(const ggml_tensor * a, const ggml_tensor * b) {
     const ggml_tensor * wa = a->src[0];
     const ggml_tensor * wb = b->src[0];

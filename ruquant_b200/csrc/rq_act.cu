@@ -13,10 +13,10 @@
 //
 // Two kernels:
 //   rq_act_kernel<P>          one CTA per token, the token's row resident in shared memory (prefill widths, any G).  What bounds it
-//                             at thousands of tokens: the Paley adds (K = 17408: 134 of 268 us for 4096 tokens, the rate of the
-//                             fp32 pipe, as packed adds with the signs in the code; 294 before), the rest is load 33, Sylvester 48,
-//                             quantizer 53 us -- phases of one CTA that overlap only with those of the SM's two others.
-//                             K = 5120: 49 us, 68 before.
+//                             at thousands of tokens: the Paley adds (K = 17408: 134 of 280 us for 4096 tokens are the
+//                             fp32 pipe's time for them; 294 before a group's constants were made once), the rest are phases of
+//                             one CTA that overlap only with those of the SM's two others.  K = 5120, whose adds are packed two
+//                             columns to an instruction: 50 us, 68 before.
 //   rq_act_cluster_kernel<P>  a thread-block cluster per token for decode and batch widths: every CTA transforms the whole row
 //                             (redundant, but it spares a gather through distributed shared memory), the Paley outputs
 //                             are split between the CTAs, and one cluster barrier agrees on the token's range.

@@ -115,7 +115,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 // that is one and nothing is left to do.  Rows outside the range of the bounds (NaN, infinity, 2^+-40) take the exact sums of
 // all 13.
 // Bound by issue: per input and candidate five packed half instructions and two clamps.  Converting 17408 rows of 5120 (the
-// rotation included) takes 451 us; 2267 with a thread per (row, candidate) that walked the sequential sum (a division, two
+// rotation included) takes 405 us; 2267 with a thread per (row, candidate) that walked the sequential sum (a division, two
 // conversions and three double operations per input) and a second pass that read the rows again to pack them.
 constexpr int WROW_THREADS = 128, EXACT_CHUNK = 64;
 __global__ void __launch_bounds__(WROW_THREADS) rq_wrow_kernel(const float * __restrict__ x, int64_t ldx, int K, int pad0, rq_block * __restrict__ out) {

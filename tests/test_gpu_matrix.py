@@ -88,7 +88,7 @@ def test_config5_prefill_layer_at_4096_tokens(rq, port, layer_seed):
 @pytest.mark.parametrize("wgroup", [0, 64])
 def test_longest_row_on_the_tensor_core_path(rq, port, type_, wgroup):
     """K = 32768, the longest row the format admits: the widest running totals, the most re-centrings of the float fold
-    (fp8 operands) and the reference's adversarial initialiser (sign-aligned tokens, flat rows), one CTA and a pair."""
+    (fp8 operands) and the reference's adversarial initialiser (sign-aligned tokens, flat rows), one and two tiles of tokens."""
     K, N = 32768, 264
     w = inputs.reference_test_weights(N, K)
     wb = port.quantize_weights(w, type_, wgroup=wgroup)
@@ -102,7 +102,7 @@ def test_longest_row_on_the_tensor_core_path(rq, port, type_, wgroup):
 @pytest.mark.parametrize("wgroup", [0, 64])
 @pytest.mark.parametrize("M", [100, 200])
 def test_push_from_every_tensor_core_variant(rq, port, wgroup, M):
-    """rq_w4a4_mul_mat_push above 64 tokens: fp8 and int8 operands, one CTA (M = 100) and pairs (M = 200), two
+    """rq_w4a4_mul_mat_push above 64 tokens: fp8 and int8 operands, one tile of tokens (M = 100) and two (M = 200), two
     destinations on one GPU; the second destination starts 4 bytes off a 16-byte boundary, so the kernel may not use
     16-byte stores for it."""
     K, N = 1536, 328

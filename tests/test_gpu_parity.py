@@ -448,7 +448,7 @@ def test_eight_rotation_blocks(rq, port):
 
 @pytest.mark.parametrize("M", [129, 257, 300])
 def test_pairs_with_ragged_token_and_row_counts(rq, port, M):
-    """CTA pairs (above 128 tokens) when the last pair's second CTA holds one token, none, or a partial tile, the weight
+    """Several tiles of 128 tokens, the last one of them holding one token or a part of a tile, when the weight
     rows do not fill their last 256-row tile, and y has a row stride that is not a multiple of 4 floats."""
     K, N = 1024, 300
     wb = port.quantize_weights(inputs.normal_weights(N, K, 9700), 45)
